@@ -309,11 +309,23 @@ void set_full_band(GridPlan &g) {
 
 }  // namespace
 
-// Shared memory of one spread / interpolation CTA: the W-plane tile of
-// (T + W - 1)^2 cells (odd row stride, plane stride 8 mod 32, real and
-// imaginary parts) and 8 warps' record staging (the layout of the device
-// kernels, GridKernels::smem_bytes).
+// Shared memory of one spread / interpolation CTA (the layouts of the device
+// kernels).  FP32: the W-plane tile of (T + W - 1)^2 cells (odd row stride,
+// plane stride 8 mod 32, real and imaginary parts) and 8 warps' record
+// staging.  FP64: the tile (plane stride 1 or 4 mod 8 cells), the staging
+// areas of 32 records, the spread's spare cells or the interpolation's sums,
+// and the records' origins.
 size_t tile_smem_bytes(int T, int W, bool fp32) {
+  if (!fp32) {
+    const size_t n = size_t(T + W - 1) * size_t(T + W - 1);
+    const size_t ps = n + ((1 + 8) - n % 8) % 8, pi = n + ((4 + 8) - n % 8) % 8;
+    const bool solo = W <= kSolo64;  // (8 warps each on their own, else two teams of 8)
+    const size_t sp = 16 * W * ps + 16 * 32 * 8 + 4 * 32 * 8 * size_t(grid64_spread_stride(W)) +
+                      4 * 128;
+    const size_t in = 16 * W * pi + (solo ? 8 : 4) * 32 * 8 * size_t(grid64_interp_stride(W)) +
+                      (solo ? 8 : 32) * 64 * 8 + (solo ? 8 : 6) * 128;
+    return std::max(sp, in);
+  }
   const size_t rs = fp32 ? 4 : 8;
   const size_t S = size_t(T + W - 1), RS = S | 1;
   size_t PS = S * RS;

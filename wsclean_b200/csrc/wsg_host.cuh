@@ -91,8 +91,14 @@ DevKernel<R> make_kernel(const PolyKernel &pk) {
   DevKernel<R> k;
   std::memset(&k, 0, sizeof(k));
   k.D = pk.D;
+  // the kernel is even, so piece W-1-i mirrors piece i: its coefficients are
+  // those of i with the odd powers negated (the fit gives the two to within
+  // rounding; their mean makes them exactly so)
   for (int j = 0; j <= pk.D; ++j)
-    for (int i = 0; i < pk.W; ++i) k.c[j][i] = R(pk.coef[size_t(j) * pk.W + i]);
+    for (int i = 0; i < pk.W; ++i) {
+      const double a = pk.coef[size_t(j) * pk.W + i], b = pk.coef[size_t(j) * pk.W + pk.W - 1 - i];
+      k.c[j][i] = R(j % 2 ? 0.5 * (a - b) : 0.5 * (a + b));
+    }
   return k;
 }
 

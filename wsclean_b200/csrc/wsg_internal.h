@@ -177,8 +177,17 @@ void limit_key_bits(GridPlan &g, int max_bits);
 std::vector<std::pair<int, double>> rank_kernels(const GridPlan &g, double sigma_min,
                                                  double sigma_max, int tile, size_t n);
 
-// Shared memory of a spread / interpolation CTA for tile T and support W.
-constexpr size_t kMaxSmemPerBlock = 227 * 1024;
+// Doubles a staged record of the FP64 spread / interpolation kernels takes
+// (wsg_grid64.cuh): a row stride of 4 mod 16 doubles.
+constexpr int grid64_pad4(int n) { return n + ((4 - n % 16) + 16) % 16; }
+constexpr int grid64_spread_stride(int W) { return grid64_pad4(8 * ((2 * W + 7) / 8) + 2 * W); }
+constexpr int grid64_interp_stride(int W) { return grid64_pad4(3 * W); }
+// Supports whose records a single warp of the interpolation handles.
+constexpr int kSolo64 = 8;
+
+// Shared memory of a spread / interpolation CTA for tile T and support W
+// (the limit leaves 1 KB to the kernels' static variables).
+constexpr size_t kMaxSmemPerBlock = 226 * 1024;
 size_t tile_smem_bytes(int T, int W, bool fp32);
 
 // The tuned schedule's subdivision (ducc0's ms2dirty_tuning / dirty2ms_tuning,

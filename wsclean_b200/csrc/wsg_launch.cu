@@ -2,6 +2,7 @@
 // support W), the pruned u transforms (over log2 M, with their staged
 // forms) and the w-screens: the one translation unit that compiles them.
 
+#include "wsg_grid64.cuh"
 #include "wsg_host.cuh"
 
 namespace wsg {
@@ -23,6 +24,7 @@ struct GridKernels {
     const size_t stage = sizeof(R) * (32 * kst + 64) + 128;  // WarpStage<R, W>::bytes
     size_t tile = ((sizeof(R) * 2 * size_t(W) * tl.PS) + 15) & ~size_t(15);
     (void)spread;
+    if (sizeof(R) == 8) return tile_smem_bytes(tl.S - W + 1, W, false);
     const size_t b = tile + size_t(NWARP) * stage;
     require(b == tile_smem_bytes(tl.S - W + 1, W, sizeof(R) == 4) && b <= kMaxSmemPerBlock,
             "internal: spread tile exceeds shared memory");
@@ -39,7 +41,11 @@ struct GridKernels {
   static void run(bool spread, dim3 grid, size_t smem, cudaStream_t st, const GridArgs &a,
                   const DevGeom &g, const DevKernel<R> &kc) {
     constexpr int P = ppl<W>();
-    if (spread) {
+    if constexpr (sizeof(R) == 8) {
+      auto fn = spread ? k_spread64<W> : k_interp64<W>;
+      smem_attr(fn, smem);
+      fn<<<grid, 32 * (spread ? Cfg64<W>::WARPS : Cfg64<W>::IWARPS), smem, st>>>(a, g, kc);
+    } else if (spread) {
       auto fn = k_spread<R, W, P, NWARP>;
       smem_attr(fn, smem);
       fn<<<grid, NWARP * 32, smem, st>>>(a, g, kc);
@@ -67,7 +73,11 @@ struct GridKernels {
     }
     constexpr int P = ppl<W>();
     int nb = 0;
-    if (spread)
+    if constexpr (sizeof(R) == 8)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spread ? k_spread64<W> : k_interp64<W>,
+                                                    32 * (spread ? Cfg64<W>::WARPS : Cfg64<W>::IWARPS),
+                                                    smem);
+    else if (spread)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_spread<R, W, P, NWARP>, NWARP * 32, smem);
     else
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_interp<R, W, P, NWARP>, NWARP * 32, smem);
@@ -85,7 +95,9 @@ struct GridKernels {
       } else {
         // set the smem attribute before asking for the occupancy
         constexpr int P = ppl<WW>();
-        if (spread)
+        if constexpr (sizeof(R) == 8)
+          smem_attr(spread ? k_spread64<WW> : k_interp64<WW>, smem);
+        else if (spread)
           smem_attr(k_spread<R, WW, P, NWARP>, smem);
         else
           smem_attr(k_interp<R, WW, P, NWARP>, smem);
@@ -344,6 +356,7 @@ int grid_groups(int W) {
 }
 template <typename R>
 bool grid_needs_acc(int W) {
+  if (sizeof(R) == 8) return false;  // (one writer a record and pass)
   const int ng = GridKernels<R>::groups(W);
   return ng > 1 && ng < GridKernels<R>::NWARP;
 }

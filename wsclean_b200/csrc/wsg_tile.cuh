@@ -1,0 +1,242 @@
+// The shared-memory tile of a spread / interpolation CTA and its exchange
+// with the band grid.  A tile holds W planes of S x S complex cells
+// (S = T + W - 1 <= 32), cell (p, ia, ib) at p PS + ia RS + ib.
+#pragma once
+
+#include "wsg_internal.h"
+// (the device header uses the host declarations above)
+#include "wsg_device.cuh"
+
+namespace wsg {
+
+// Adding to a shared-memory cell that other warps may be adding to, without a
+// lock or a compare-and-swap loop: take() empties the cell, put() puts the sum
+// back and returns what a concurrent add left there in between (zero as a
+// rule), which the caller adds in turn.  Of two adds that collide at least one
+// is done, so the loop ends.  Exchanges run at the rate of plain loads and
+// stores (2.1 cycles a warp for 64 bits on the B200), FP32 and FP64
+// shared-memory additions at 6 to 11 cycles a warp.
+__device__ __forceinline__ unsigned long long exch64(void *p, unsigned long long v) {
+  return atomicExch(reinterpret_cast<unsigned long long *>(p), v);
+}
+__device__ __forceinline__ double take(double *p) {
+  return __longlong_as_double((long long)exch64(p, 0ull));
+}
+__device__ __forceinline__ double put(double *p, double v) {
+  return __longlong_as_double((long long)exch64(p, (unsigned long long)__double_as_longlong(v)));
+}
+
+// The cells of a chunk's tile that its records touch, as lines along v: over
+// the bounding box of the footprints, or footprint by footprint when few
+// origins were used.  A warp takes up to 32 consecutive lines at a time: each
+// lane finds one line's grid row, then the warp walks the lines with lanes
+// along v (several short lines side by side), so that finding a row costs one
+// lane's work instead of a warp's (the flush and the staging of a W = 8 tile
+// of 27 x 27 cells took 70 warp instructions a line when every lane did it).
+struct TileLines {
+  int nline, len, lpi, sub, col, gsz;
+  bool by_list, act;
+  int lu0, lv0, nbu;
+  const uint32_t *orig;
+};
+
+template <int W>
+__device__ __forceinline__ TileLines tile_lines(const int *bb, int norig, const uint32_t *orig,
+                                                int lane, int nwarp) {
+  TileLines t;
+  t.lu0 = bb[0];
+  t.lv0 = bb[2];
+  t.nbu = max(bb[1] + W - t.lu0, 0);
+  const int nbv = max(bb[3] + W - t.lv0, 0);
+  t.by_list = norig <= kMaxOrig && norig * W * W < t.nbu * nbv;
+  t.nline = t.by_list ? norig * W * W : W * t.nbu;
+  t.len = t.by_list ? W : max(nbv, 1);
+  t.lpi = 32 / t.len;
+  t.sub = lane / t.len;
+  t.col = lane - t.sub * t.len;
+  t.act = t.sub < t.lpi;
+  t.gsz = min(32, (t.nline + nwarp - 1) / nwarp);
+  t.orig = orig;
+  return t;
+}
+
+// One lane's line: its tile offset, the grid row (null outside the pass or
+// the band) and the first v index.
+template <int W, typename C>
+__device__ __forceinline__ C *tile_line(const TileLines &t, const JobRegs &jr, int line, int mp,
+                                        int ucorner, int vcorner, int RS, int PS, uint32_t &where) {
+  int p, ia, ib;
+  if (t.by_list) {
+    const int o = line / (W * W), pr = line - o * W * W;
+    p = pr / W;
+    const uint32_t luv = t.orig[o];
+    ia = int(luv >> 16) + (pr - p * W);
+    ib = int(luv & 0xffffu);
+  } else {
+    p = line / t.nbu;
+    ia = t.lu0 + (line - p * t.nbu);
+    ib = t.lv0;
+  }
+  where = (uint32_t(jr.wrap_v(vcorner + ib)) << 16) | uint32_t(p * PS + ia * RS + ib);
+  const int plane = mp + p;
+  const int bi = jr.band_row(jr.wrap_u(ucorner + ia));
+  if (plane < jr.pb0 || plane >= jr.pb1 || bi < 0) return nullptr;
+  return reinterpret_cast<C *>(jr.grid) + (size_t(bi) * jr.P + (plane - jr.pb0)) * size_t(jr.nv);
+}
+
+__device__ __forceinline__ void *shfl_ptr(void *p, int src) {
+  return reinterpret_cast<void *>(
+      __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), src));
+}
+
+__device__ __forceinline__ float2 take_cell(float2 *p) {
+  const unsigned long long v = exch64(p, 0ull);
+  return make_float2(__uint_as_float(uint32_t(v)), __uint_as_float(uint32_t(v >> 32)));
+}
+__device__ __forceinline__ double2 take_cell(double2 *p) {
+  return make_double2(take(&p->x), take(&p->y));
+}
+__device__ __forceinline__ void red_cell(float2 *p, float2 v) { atomicAdd(p, v); }
+__device__ __forceinline__ void red_cell(double2 *p, double2 v) {
+  atomicAdd(&p->x, v.x);
+  atomicAdd(&p->y, v.y);
+}
+
+// Adds the touched cells of the tile to the band grid and leaves them zero
+// (a cell shared by two listed footprints is taken once).
+template <int W, typename C>
+__device__ __forceinline__ void tile_flush(C *tile, int RS, int PS, const TileLines &t,
+                                           const JobGeom &jb, int mp, int ucorner, int vcorner,
+                                           int warp, int lane, int nwarp) {
+  const JobRegs jr(jb);
+  for (int l0 = warp * t.gsz; l0 < t.nline; l0 += nwarp * t.gsz) {
+    uint32_t where = 0;
+    C *row = nullptr;
+    if (lane < t.gsz && l0 + lane < t.nline)
+      row = tile_line<W, C>(t, jr, l0 + lane, mp, ucorner, vcorner, RS, PS, where);
+    const int n = min(t.gsz, t.nline - l0);
+    for (int i = 0; i < n; i += t.lpi) {
+      const int src = min(i + t.sub, 31);
+      C *const rp = reinterpret_cast<C *>(shfl_ptr(row, src));
+      const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
+      if (t.act && i + t.sub < n) {
+        const C x = take_cell(&tile[(wh & 0xffffu) + t.col]);
+        if (rp && (x.x != 0 || x.y != 0)) {
+          int v = int(wh >> 16) + t.col;
+          v -= v >= jr.nv ? jr.nv : 0;
+          red_cell(rp + v, x);
+        }
+      }
+    }
+  }
+}
+
+// Reads the touched cells from the band grid, eight lines in flight; store
+// (tile offset, value) puts one cell into the tile.
+template <int W, typename C, typename Store>
+__device__ __forceinline__ void tile_stage(int RS, int PS, const TileLines &t, const JobGeom &jb,
+                                           int mp, int ucorner, int vcorner, int warp, int lane,
+                                           int nwarp, Store &&store) {
+  const JobRegs jr(jb);
+  for (int l0 = warp * t.gsz; l0 < t.nline; l0 += nwarp * t.gsz) {
+    uint32_t where = 0;
+    C *row = nullptr;
+    if (lane < t.gsz && l0 + lane < t.nline)
+      row = tile_line<W, C>(t, jr, l0 + lane, mp, ucorner, vcorner, RS, PS, where);
+    const int n = min(t.gsz, t.nline - l0);
+    for (int i0 = 0; i0 < n; i0 += 8 * t.lpi) {
+      C val[8];
+      int at[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int i = i0 + q * t.lpi, src = min(i + t.sub, 31);
+        const C *const rp = reinterpret_cast<const C *>(shfl_ptr(row, src));
+        const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
+        val[q].x = val[q].y = 0;
+        at[q] = -1;
+        if (t.act && i + t.sub < n) {
+          at[q] = int(wh & 0xffffu) + t.col;
+          if (rp) {
+            int v = int(wh >> 16) + t.col;
+            v -= v >= jr.nv ? jr.nv : 0;
+            val[q] = rp[v];
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (at[q] >= 0) store(at[q], val[q]);
+    }
+  }
+}
+
+// The chunk a CTA works on (read by thread 0 into shared memory).
+struct ChunkState {
+  int chunk, norig;
+  int bb[4];
+  uint32_t orig[kMaxOrig];
+  JobGeom job;
+};
+
+__device__ __forceinline__ void next_chunk(ChunkState &cs, const GridArgs &a, const DevGeom &g) {
+  cs.chunk = atomicAdd(a.counter, 1);
+  cs.bb[0] = cs.bb[2] = 1 << 30;
+  cs.bb[1] = cs.bb[3] = -1;
+  cs.norig = 0;
+  if (cs.chunk < *a.nchunks) cs.job = load_job(a, g, cs.chunk);
+}
+
+// Lists a staged batch's new footprint origins (one warp): my is the lane's
+// packed origin, prev the last one of the batch before.  A repeated origin in
+// the list is harmless, its cells being taken once.
+__device__ __forceinline__ void list_origins(ChunkState &cs, uint32_t my, bool valid, uint32_t prev,
+                                             int lane) {
+  uint32_t before = __shfl_up_sync(0xffffffffu, my, 1);
+  if (lane == 0) before = prev;
+  const unsigned nm = __ballot_sync(0xffffffffu, valid && my != before && my != kSkip);
+  if (!nm) return;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(&cs.norig, __popc(nm));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  const int k = base + __popc(nm & ((1u << lane) - 1u));
+  if (((nm >> lane) & 1u) && k < kMaxOrig) cs.orig[k] = my;
+}
+
+// Bounding box of the lanes' origins into the chunk's (one warp).
+__device__ __forceinline__ void merge_box(ChunkState &cs, int b0, int b1, int b2, int b3, int lane) {
+  b0 = __reduce_min_sync(0xffffffffu, b0);
+  b1 = __reduce_max_sync(0xffffffffu, b1);
+  b2 = __reduce_min_sync(0xffffffffu, b2);
+  b3 = __reduce_max_sync(0xffffffffu, b3);
+  if (lane == 0 && b1 >= 0) {
+    atomicMin(&cs.bb[0], b0);
+    atomicMax(&cs.bb[1], b1);
+    atomicMin(&cs.bb[2], b2);
+    atomicMax(&cs.bb[3], b3);
+  }
+}
+
+// Bounding box and distinct origins of a chunk's records [s0, s1), by all
+// warps (before an interpolation stages its tile).
+template <typename Rec>
+__device__ __forceinline__ void scan_origins(ChunkState &cs, const Rec *recs, int s0, int s1, int tu,
+                                             int tv, int T, int tid, int nthr) {
+  const int lane = tid & 31;
+  int b0 = 1 << 30, b1 = -1, b2 = 1 << 30, b3 = -1;
+  for (int s = s0 + tid - lane; s < s1; s += nthr) {
+    uint32_t luv = kSkip;
+    if (s + lane < s1) {
+      const uint32_t iuv = recs[s + lane].iuv;
+      const int lu = int(iuv >> 16) - tu * T, lv = int(iuv & 0xffffu) - tv * T;
+      if (lu >= 0 && lu < T && lv >= 0 && lv < T) {
+        luv = (uint32_t(lu) << 16) | uint32_t(lv);
+        b0 = min(b0, lu); b1 = max(b1, lu);
+        b2 = min(b2, lv); b3 = max(b3, lv);
+      }
+    }
+    list_origins(cs, luv, true, kSkip, lane);
+  }
+  merge_box(cs, b0, b1, b2, b3, lane);
+}
+
+}  // namespace wsg
