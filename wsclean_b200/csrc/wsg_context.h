@@ -156,7 +156,8 @@ class Context {
   cudaStream_t stream = nullptr, own_stream = nullptr;
   int num_sms = 148;
   int verbosity = 0;
-  int chunk_size = 2048;  // records per chunk at most (a bin may take several)
+  // records per chunk at most (a bin may take several), and the limit's range
+  static constexpr int chunk_min = 64, chunk_max = 2048;
   wsg_stats stats;
   double cheb_err = 0;
 

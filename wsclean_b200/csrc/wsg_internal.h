@@ -151,6 +151,8 @@ struct GridPlan {
   // batch plans: every job uses the kernel (W, sigma) of the first one
   int force_W = 0;
   double force_sigma = 0;
+  // a batch plan's job: its chunks share their launches with the other jobs'
+  bool batch = false;
   // streams: the grid was planned from a declared data extent; chunks are
   // checked against it instead of re-planning
   bool fixed = false;

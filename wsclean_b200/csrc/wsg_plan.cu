@@ -153,6 +153,7 @@ void Plan::build(const std::vector<wsg_job> &js) {
     gp.mshift = a_.negate_v ? -jd.center_y : jd.center_y;
     gp.force_W = forceW;
     gp.force_sigma = forceS;
+    gp.batch = jobs_.size() > 1;
     const bool any = cx_.prepare<R>(aj, sj, false, nullptr, gp);
     if (forceW == 0 && any) {  // the largest job with active visibilities
       forceW = gp.kernel.W;
