@@ -310,29 +310,25 @@ void set_full_band(GridPlan &g) {
 }  // namespace
 
 // Shared memory of one spread / interpolation CTA (the layouts of the device
-// kernels).  FP32: the W-plane tile of (T + W - 1)^2 cells (odd row stride,
-// plane stride 8 mod 32, real and imaginary parts) and 8 warps' record
-// staging.  FP64: the tile (plane stride 1 or 4 mod 8 cells), the staging
-// areas of 32 records, the spread's spare cells or the interpolation's sums,
-// and the records' origins.
+// kernels, the larger of the two directions).  FP32: the W-plane tile of
+// (T + W - 1)^2 cells (odd row stride, plane stride 8 mod 16) and each
+// warp's staging area of 32 records.  FP64: the tile (plane stride 1 or 4 mod
+// 8 cells), the staging areas of 32 records, the spread's spare cells or the
+// interpolation's sums, and the records' origins.
 size_t tile_smem_bytes(int T, int W, bool fp32) {
-  if (!fp32) {
-    const size_t n = size_t(T + W - 1) * size_t(T + W - 1);
-    const size_t ps = n + ((1 + 8) - n % 8) % 8, pi = n + ((4 + 8) - n % 8) % 8;
-    const bool solo = W <= kSolo64;  // (8 warps each on their own, else two teams of 8)
-    const size_t sp = 16 * W * ps + 16 * 32 * 8 + 4 * 32 * 8 * size_t(grid64_spread_stride(W)) +
-                      4 * 128;
-    const size_t in = 16 * W * pi + (solo ? 8 : 4) * 32 * 8 * size_t(grid64_interp_stride(W)) +
-                      (solo ? 8 : 32) * 64 * 8 + (solo ? 8 : 6) * 128;
-    return std::max(sp, in);
+  const size_t S = size_t(T + W - 1);
+  if (fp32) {
+    const size_t n = S * (S | 1), ps = n + (8 + 16 - n % 16) % 16;
+    return 8 * W * ps + kGrid32Warps * 32 * 4 * size_t(std::max(36, grid32_stride(W)));
   }
-  const size_t rs = fp32 ? 4 : 8;
-  const size_t S = size_t(T + W - 1), RS = S | 1;
-  size_t PS = S * RS;
-  PS += ((8 - (PS % 32)) + 32) % 32;
-  const size_t kst = fp32 ? ((3 * size_t(W) + 3) & ~size_t(3)) : ((3 * size_t(W) + 1) & ~size_t(1));
-  const size_t stage = rs * (32 * kst + 64) + 128;
-  return ((rs * 2 * size_t(W) * PS + 15) & ~size_t(15)) + 8 * stage;
+  const size_t n = S * S;
+  const size_t ps = n + ((1 + 8) - n % 8) % 8, pi = n + ((4 + 8) - n % 8) % 8;
+  const bool solo = W <= kSolo64;  // (8 warps each on their own, else two teams of 8)
+  const size_t sp = 16 * W * ps + 16 * 32 * 8 + 4 * 32 * 8 * size_t(grid64_spread_stride(W)) +
+                    4 * 128;
+  const size_t in = 16 * W * pi + (solo ? 8 : 4) * 32 * 8 * size_t(grid64_interp_stride(W)) +
+                    (solo ? 8 : 32) * 64 * 8 + (solo ? 8 : 6) * 128;
+  return std::max(sp, in);
 }
 
 // nu = K * 2^m with 2^m >= 2L+1, so that the occupied u band fits one pruned

@@ -60,10 +60,10 @@ int env_int(const char *name, int dflt) {
 }
 
 // Bin tile edge asked of the planner (which shrinks it until the W-plane
-// tile fits shared memory): measured on the 8.1M-visibility 4096^2 pair,
-// 20 is the fastest in mixed precision (3 -> 2 CTAs per SM, but half the
-// tile flushes of 16) and 24 in FP64; WSG_TILE overrides it.
-int default_tile(bool fp32) { return env_int("WSG_TILE", fp32 ? 20 : 24); }
+// tile fits shared memory).  Measured on the 8.1M-visibility 4096^2 pair: in
+// mixed precision 24 is 6% faster than 20 and 17% than 16 in both kernels (two
+// CTAs an SM each way); WSG_TILE overrides it.
+int default_tile(bool) { return env_int("WSG_TILE", 24); }
 
 // --------------------------------------------------------------- context
 
@@ -720,8 +720,6 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
   ColArgs ca{};
   if (!gp.ucufft) ca = make_col(gp, P, upload_twiddles(gp, dbl), bandf, H);
   const long Lv = band_v_halfwidth(gp);
-  const TileLayout tl = make_layout(gp.T, gp.kernel.W);
-  const size_t smem = grid_smem_bytes<R>(tl, gp.kernel.W, true);
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
@@ -735,8 +733,6 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
   ga.nvis = int(gp.nvis);
   ga.grid = band;
   ga.P = int(P);
-  ga.tl = tl;
-  ga.sb = grid_sb<R>();
 
   const int dir = CUFFT_INVERSE;
   float t_grid = 0, t_fft = 0, t_screen = 0;
@@ -747,7 +743,7 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
     CK(cudaMemsetAsync(counter, 0, sizeof(int), stream));
     ga.pb0 = int(pb0);
     ga.pb1 = int(pb0 + npl);
-    grid_dispatch<R>(gp.kernel.W, true, num_sms, smem, stream, ga, g, kc);
+    grid_dispatch<R>(gp.kernel.W, true, num_sms, stream, ga, g, kc);
     band_dirty = BandDirty{band, rowsP, nv, cs, Lv};
     CK(cudaEventRecord(ev[3], stream));
     if (gp.ucufft) {
@@ -846,8 +842,6 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
   char *H = gp.ucufft ? nullptr : reinterpret_cast<char *>(b_H.ensure(P * gp.ny * gp.hrow() * cs));
   ColArgs ca{};
   if (!gp.ucufft) ca = make_col(gp, P, upload_twiddles(gp, dbl), bandi, H);
-  const TileLayout tl = make_layout(gp.T, gp.kernel.W);
-  const size_t smem = grid_smem_bytes<R>(tl, gp.kernel.W, false);
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
@@ -861,13 +855,10 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
   ga.nvis = int(gp.nvis);
   ga.grid = band;
   ga.P = int(P);
-  ga.tl = tl;
-  ga.sb = grid_sb<R>();
   ga.vis_out = vis_out;
   ga.vis_double = a.vis_type == WSG_C128;
   ga.vis_accumulate = vis_acc ? 1 : 0;
-  const bool multi = P < gp.nplanes;
-  const bool need_acc = multi || grid_needs_acc<R>(gp.kernel.W);
+  const bool need_acc = P < gp.nplanes;  // sums over several plane passes
   ga.acc = need_acc ? b_acc.ensure(gp.nvis * cs) : nullptr;
   if (need_acc) CK(cudaMemsetAsync(ga.acc, 0, gp.nvis * cs, stream));
 
@@ -915,7 +906,7 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
     ga.pb1 = int(pb0 + npl);
     ga.first_pass = pb0 == 0;
     ga.last_pass = pb0 + npl >= gp.nplanes;
-    grid_dispatch<R>(gp.kernel.W, false, num_sms, smem, stream, ga, g, kc);
+    grid_dispatch<R>(gp.kernel.W, false, num_sms, stream, ga, g, kc);
     CK(cudaEventRecord(ev[5], stream));
     float t = 0;
     if (!async_mode) CK(cudaEventSynchronize(ev[5]));

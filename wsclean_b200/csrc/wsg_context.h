@@ -300,13 +300,12 @@ class Plan {
   wsg_args a_;
   bool dbl_ = false;
   std::vector<PlanJob> jobs_;
-  DevBuf rec_, chunks_, chunk_job_, jobgeom_, band_, H_, img_, cf_, tw_, acc_, small_, fftwork_;
+  DevBuf rec_, chunks_, chunk_job_, jobgeom_, band_, H_, img_, cf_, tw_, small_, fftwork_;
   size_t nrec_ = 0, band_total_ = 0, max_npix_ = 0;
   int nchunks_ = 0;
   std::vector<unsigned char> kernel_;  // DevKernel<R> bytes
   std::vector<unsigned char> geom_;    // DevGeom of the first job (kernel, tile: shared)
   int W_ = 0, T_ = 0;
-  bool need_acc_ = false;
   // graphs recorded per (mode, pointers, accumulate)
   struct Graph {
     int mode = 0, accumulate = 0;

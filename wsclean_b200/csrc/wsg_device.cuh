@@ -9,7 +9,8 @@
 //   visibility in key order with FP64 pixel coordinates reduced to local kernel
 //   coordinates and the shift phasor / weight / conjugation applied
 //                                                             (compute_phases, wgridder.h:1126-1140)
-//   k_spread    persistent CTAs drain chunks of one (tile, minplane) bin each,
+//   k_spread32 / k_spread64 (wsg_grid32.cuh, wsg_grid64.cuh)
+//               persistent CTAs drain chunks of one (tile, minplane) bin each,
 //               accumulate W planes x W x W footprints in registers while the
 //               footprint origin repeats, commit to a shared-memory tile, and
 //               flush the tile to the u-band grid with vector atomics
@@ -213,13 +214,6 @@ __device__ __forceinline__ double weighted(const ImgW &iw, const double *__restr
                        : 0.0;
   const double p = w * f;
   return sizeof(TW) == 4 ? double(float(p)) : p;
-}
-
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
 }
 
 // --------------------------------------------------------------- k_scan
@@ -468,13 +462,7 @@ struct ChunkStartPred {
   }
 };
 
-// ------------------------------------------------------- tile geometry
-
-struct TileLayout {
-  int S;    // tile extent incl. halo: T + W - 1
-  int RS;   // row stride (elements), odd
-  int PS;   // plane stride (elements)
-};
+// ------------------------------------------------------- gridding jobs
 
 // Grid geometry of one gridding job.  A call is one job; a batch plan runs
 // many jobs (facets x output channels) sharing one kernel, tile size and
@@ -494,8 +482,6 @@ struct GridArgs {
   void *grid;        // u-band grid [band_rows][P][nv] complex
   int P;             // planes in the layout
   int pb0, pb1;      // planes of this pass: [pb0, pb1)
-  TileLayout tl;
-  int sb;            // records per sub-batch
   int *err;          // set to 1 if a record falls outside its chunk's tile
   // degridding outputs
   void *vis_out;     // complex TV
@@ -557,496 +543,16 @@ struct JobRegs {
 };
 
 constexpr uint32_t kSkip = 0xfffffffeu;  // record marker: outside its chunk's tile
+constexpr uint32_t kNone = 0xffffffffu;  // no origin yet
 
 
-// ------------------------------------------------- per-warp record staging
-//
-// A warp works through its slice of a chunk 32 records at a time: lane l
-// loads record l of the batch (coalesced), evaluates its 3W kernel values --
-// W pieces per axis by Horner's rule of fixed degree W+4 with the
-// coefficients as compile-time constant-bank operands (the host pads
-// lower-degree fits with zero leading coefficients) -- and stages them in a
-// per-warp shared-memory block; the warp then consumes the batch record by
-// record with broadcast reads.
+// Degree of the kernel polynomials the device evaluates (the host pads
+// lower-degree fits with zero leading coefficients).
 template <int W> struct KDeg { static constexpr int value = W + 4; };
-template <typename R, int W> struct KStride {
-  // row of 3W values, padded to a 16-byte multiple
-  static constexpr int value = sizeof(R) == 4 ? ((3 * W + 3) & ~3) : ((3 * W + 1) & ~1);
-};
-template <typename R, int W> struct WarpStage {
-  static constexpr int KST = KStride<R, W>::value;
-  static constexpr size_t bytes = sizeof(R) * (32 * KST + 64) + 128;  // kv, (vr,vi), luv
-};
-
-// W consecutive values of a staged row, by 16- or 8-byte vector loads where
-// the layout allows: with W even every staged row, and its v block at W,
-// starts on a 16-byte boundary (the tile before the staging areas holds
-// 2 W planes, and the row stride is a multiple of 16 bytes).
-template <int W, typename R>
-__device__ __forceinline__ void lds_row(const R *p, R (&out)[W]) {
-  if constexpr (sizeof(R) == 4 && W % 4 == 0) {
-#pragma unroll
-    for (int i = 0; i < W / 4; ++i) {
-      const float4 v = reinterpret_cast<const float4 *>(p)[i];
-      out[4 * i] = v.x;
-      out[4 * i + 1] = v.y;
-      out[4 * i + 2] = v.z;
-      out[4 * i + 3] = v.w;
-    }
-  } else if constexpr (W % 2 == 0) {
-    using V2 = typename Cplx<R>::type;
-#pragma unroll
-    for (int i = 0; i < W / 2; ++i) {
-      const V2 v = reinterpret_cast<const V2 *>(p)[i];
-      out[2 * i] = v.x;
-      out[2 * i + 1] = v.y;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) out[i] = p[i];
-  }
-}
-
-template <int W, typename R>
-__device__ __forceinline__ void eval_const(const DevKernel<R> &k, R x, R *out) {
-  constexpr int DEG = KDeg<W>::value;
-#pragma unroll
-  for (int i = 0; i < W; ++i) {
-    R v = k.c[DEG][i];
-#pragma unroll
-    for (int j = DEG - 1; j >= 0; --j) v = fma(v, x, k.c[j][i]);
-    out[i] = v;
-  }
-}
-
-// The per-record part of staging that is not kernel evaluation: the packed
-// in-tile origin (or kSkip when the record lies outside its chunk's tile),
-// the bounding box of origins, and the visibility to spread (gathered and
-// multiplied by the static factor for plan execution).  Returns false for a
-// skipped record.
-template <typename R, typename Rec>
-__device__ __forceinline__ bool stage_meta(const Rec &rr, int lane, int tu, int tv, int mp,
-                                           const DevGeom &g, R *vv, uint32_t *luv, int *err,
-                                           int &bb0, int &bb1, int &bb2, int &bb3,
-                                           const void *vis_in, int vis_in_double) {
-  const int lu = int(rr.iuv >> 16) - tu * g.T;
-  const int lv = int(rr.iuv & 0xffffu) - tv * g.T;
-  if (lu < 0 || lu >= g.T || lv < 0 || lv >= g.T || int(rr.mp) != mp) {
-    atomicOr(err, 1);
-    luv[lane] = kSkip;
-    vv[2 * lane] = R(0);
-    vv[2 * lane + 1] = R(0);
-    return false;
-  }
-  luv[lane] = (uint32_t(lu) << 16) | uint32_t(lv);
-  bb0 = min(bb0, lu); bb1 = max(bb1, lu);
-  bb2 = min(bb2, lv); bb3 = max(bb3, lv);
-  R vr = rr.vr, vi = rr.vi;
-  if (vis_in) {
-    const uint32_t id = rr.idx & 0x7fffffffu;
-    R xr, xi;
-    if (vis_in_double) {
-      const double2 x = reinterpret_cast<const double2 *>(vis_in)[id];
-      xr = R(x.x);
-      xi = R(x.y);
-    } else {
-      const float2 x = reinterpret_cast<const float2 *>(vis_in)[id];
-      xr = R(x.x);
-      xi = R(x.y);
-    }
-    vr = xr * rr.vr + xi * rr.vi;
-    vi = xi * rr.vr - xr * rr.vi;
-    if (rr.idx & 0x80000000u) vi = -vi;
-  }
-  vv[2 * lane] = vr;
-  vv[2 * lane + 1] = vi;
-  return true;
-}
-
-// Stages records [b0, b0+nb) of the warp's slice; returns via luv the packed
-// in-tile origin (or kSkip).  Lanes >= nb do nothing.
-template <typename R, int W, typename Rec>
-__device__ __forceinline__ void stage_batch(const Rec *recs, int b0, int nb, int lane, int tu,
-                                            int tv, int mp, const DevGeom &g,
-                                            const DevKernel<R> &kc, R *kv, R *vv, uint32_t *luv,
-                                            int *err, int &bb0, int &bb1, int &bb2, int &bb3,
-                                            const void *vis_in, int vis_in_double) {
-  constexpr int KST = KStride<R, W>::value;
-  if (lane < nb) {
-    const Rec rr = recs[b0 + lane];
-    R *row = kv + lane * KST;
-    if (!stage_meta<R>(rr, lane, tu, tv, mp, g, vv, luv, err, bb0, bb1, bb2, bb3, vis_in,
-                       vis_in_double)) {
-#pragma unroll
-      for (int i = 0; i < 3 * W; ++i) row[i] = R(0);
-    } else {
-      R vals[W];
-      eval_const<W>(kc, rr.xu, vals);
-#pragma unroll
-      for (int i = 0; i < W; ++i) row[i] = vals[i];
-      eval_const<W>(kc, rr.xv, vals);
-#pragma unroll
-      for (int i = 0; i < W; ++i) row[W + i] = vals[i];
-      if (g.do_w) {
-        eval_const<W>(kc, rr.xw, vals);
-#pragma unroll
-        for (int i = 0; i < W; ++i) row[2 * W + i] = vals[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < W; ++i) row[2 * W + i] = R(i == 0);
-      }
-    }
-  }
-}
-
-// Staging shared by all NW warps of a CTA that works as one slice (large W
-// in FP64): lane l of warp w evaluates kernel values [w Q, (w + 1) Q) of the
-// 3W of record l (Q = ceil(3W / NW)), instead of every warp evaluating all of
-// them; warp 0 also does the rest of the staging.  The caller brackets it
-// with CTA barriers.
-template <typename R, int W, int NW, typename Rec>
-__device__ __forceinline__ void stage_batch_split(const Rec *recs, int b0, int nb, int lane, int w,
-                                                  int tu, int tv, int mp, const DevGeom &g,
-                                                  const DevKernel<R> &kc, R *kv, R *vv,
-                                                  uint32_t *luv, int *err, int &bb0, int &bb1,
-                                                  int &bb2, int &bb3, const void *vis_in,
-                                                  int vis_in_double) {
-  constexpr int KST = KStride<R, W>::value;
-  constexpr int Q = (3 * W + NW - 1) / NW;
-  constexpr int DEG = KDeg<W>::value;
-  if (lane < nb) {
-    const Rec rr = recs[b0 + lane];
-    if (w == 0)
-      stage_meta<R>(rr, lane, tu, tv, mp, g, vv, luv, err, bb0, bb1, bb2, bb3, vis_in,
-                    vis_in_double);
-    R *row = kv + lane * KST;
-#pragma unroll
-    for (int qi = 0; qi < Q; ++qi) {
-      const int v = w * Q + qi;  // the same for every lane of the warp
-      if (v < 3 * W) {
-        const int axis = v / W, piece = v - axis * W;
-        R val;
-        if (axis == 2 && !g.do_w) {
-          val = R(piece == 0);
-        } else {
-          const R x = axis == 0 ? rr.xu : (axis == 1 ? rr.xv : rr.xw);
-          val = kc.c[DEG][piece];
-#pragma unroll
-          for (int j = DEG - 1; j >= 0; --j) val = fma(val, x, kc.c[j][piece]);
-        }
-        row[v] = val;
-      }
-    }
-  }
-}
-
-// Warps sharing one record's footprint: when more than half the warps would,
-// all of them do, as one slice whose warps also share the record staging.
-template <int W, int PPL, int NWARP>
-struct WarpGroups {
-  static constexpr int NG0 = (W * W + 32 * PPL - 1) / (32 * PPL);
-  static constexpr int NG = NG0 > NWARP / 2 ? NWARP : NG0;
-  static constexpr int NSL = NWARP / NG;
-  static constexpr bool SPLIT = (NG == NWARP) && NG > 1;
-};
-
-// Warp sums of G complex values at once (G = 1, 2, 4 or 8), as a
-// reduce-scatter: at each of the first log2(G) butterfly stages a lane keeps
-// the half of its values that its lane bit names and adds the partner's
-// copy of that half, so G sums cost about 2G + 2 log2(32/G) shuffles instead
-// of 10 G.  On return every lane holds the total of value
-// (lane >> (5 - log2 G)) & (G - 1).
-template <int G, typename C>
-__device__ __forceinline__ C warp_sum_scatter(C (&v)[G], int lane) {
-  constexpr int LG = G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3;
-  static_assert((1 << LG) == G, "warp_sum_scatter: G must be 1, 2, 4 or 8");
-#pragma unroll
-  for (int st = 0; st < LG; ++st) {
-    const int b = 4 - st;
-    const int n = G >> st;  // values held before this stage
-    const bool hi = (lane >> b) & 1;
-#pragma unroll
-    for (int i = 0; i < n / 2; ++i) {
-      C send = hi ? v[i] : v[n / 2 + i];
-      const C keep = hi ? v[n / 2 + i] : v[i];
-      send.x = __shfl_xor_sync(0xffffffffu, send.x, 1 << b);
-      send.y = __shfl_xor_sync(0xffffffffu, send.y, 1 << b);
-      v[i] = cadd(keep, send);
-    }
-  }
-  C t = v[0];
-#pragma unroll
-  for (int b = 4 - LG; b >= 0; --b) {
-    t.x += __shfl_xor_sync(0xffffffffu, t.x, 1 << b);
-    t.y += __shfl_xor_sync(0xffffffffu, t.y, 1 << b);
-  }
-  return t;
-}
-
-__device__ __forceinline__ void warp_minmax(int &bb0, int &bb1, int &bb2, int &bb3) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    bb0 = min(bb0, __shfl_xor_sync(0xffffffffu, bb0, o));
-    bb1 = max(bb1, __shfl_xor_sync(0xffffffffu, bb1, o));
-    bb2 = min(bb2, __shfl_xor_sync(0xffffffffu, bb2, o));
-    bb3 = max(bb3, __shfl_xor_sync(0xffffffffu, bb3, o));
-  }
-}
-
-// ------------------------------------------------------------- k_spread
-//
-// Persistent CTAs drain chunks; all records of a chunk share one
-// (tile, minplane) bin, so the CTA owns a W-plane shared-memory tile
-// (structure of arrays: real parts, then imaginary parts) for the chunk.  Each
-// warp takes a contiguous slice of the chunk; lane q owns PPL (plane, u-row)
-// pairs of the footprint and the W cells along v of each, accumulating in
-// registers while consecutive records share the footprint origin (records are
-// sorted by position inside the tile), then commits with shared-memory
-// atomics.  At the end of the chunk the touched region is added to the u-band
-// grid with vector atomics.
-// Atomically reads a shared-memory cell and leaves zero in it.
-__device__ __forceinline__ float take_zero(float *p) { return atomicExch(p, 0.0f); }
-__device__ __forceinline__ double take_zero(double *p) {
-  return __longlong_as_double(
-      (long long)atomicExch(reinterpret_cast<unsigned long long *>(p), 0ull));
-}
 
 // Chunks touching few distinct footprint origins are flushed / staged
 // footprint by footprint instead of over their bounding box.
 constexpr int kMaxOrig = 64;
-
-template <typename R, int W, int PPL, int NWARP>
-__global__ void __launch_bounds__(NWARP * 32, sizeof(R) == 4 ? 3 : 1)
-k_spread(GridArgs a, DevGeom g, DevKernel<R> kc) {
-  using Rec = typename RecOf<R>::type;
-  using C = typename Cplx<R>::type;
-  constexpr int NG = WarpGroups<W, PPL, NWARP>::NG;    // warps per record
-  constexpr int NSL = WarpGroups<W, PPL, NWARP>::NSL;  // record slices
-  constexpr bool SPLIT = WarpGroups<W, PPL, NWARP>::SPLIT;
-  constexpr int KST = KStride<R, W>::value;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const TileLayout tl = a.tl;
-  R *tre = reinterpret_cast<R *>(smem_raw);
-  R *tim = tre + W * tl.PS;
-  __shared__ int sh_chunk, sh_bb[4], sh_norig;
-  __shared__ uint32_t sh_orig[kMaxOrig];
-  __shared__ JobGeom sh_job;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int grp = warp % NG, slice = warp / NG;
-  // the warp's own staging area, and the one it reads records from (warp 0's
-  // when the CTA's warps share the staging)
-  unsigned char *wown = smem_raw + size_t(2 * W * tl.PS) * sizeof(R) + warp * WarpStage<R, W>::bytes;
-  unsigned char *wbase = SPLIT ? smem_raw + size_t(2 * W * tl.PS) * sizeof(R) : wown;
-  R *kv = reinterpret_cast<R *>(wbase);
-  R *vv = kv + 32 * KST;
-  uint32_t *luvs = reinterpret_cast<uint32_t *>(vv + 64);
-  const Rec *recs = reinterpret_cast<const Rec *>(a.rec);
-
-  for (int i = tid; i < 2 * W * tl.PS; i += blockDim.x) tre[i] = R(0);
-  int pp[PPL], cu[PPL];
-#pragma unroll
-  for (int k = 0; k < PPL; ++k) {
-    const int q = grp * 32 * PPL + lane + 32 * k;
-    pp[k] = q / W;
-    cu[k] = q - pp[k] * W;
-  }
-
-  for (;;) {
-    __syncthreads();
-    if (tid == 0) {
-      sh_chunk = atomicAdd(a.counter, 1);
-      sh_bb[0] = 1 << 30; sh_bb[1] = -1; sh_bb[2] = 1 << 30; sh_bb[3] = -1;
-      sh_norig = 0;
-      if (sh_chunk < *a.nchunks) sh_job = load_job(a, g, sh_chunk);
-    }
-    __syncthreads();
-    const int ch = sh_chunk;
-    if (ch >= *a.nchunks) break;
-    const JobGeom &jb = sh_job;  // read from shared memory where used
-    const int s0 = a.chunk_start[ch];
-    const int s1 = (ch + 1 < *a.nchunks) ? a.chunk_start[ch + 1] : a.nvis;
-    const Rec r0 = recs[s0];
-    const int tu = int(r0.iuv >> 16) / g.T, tv = int(r0.iuv & 0xffffu) / g.T;
-    const int mp = int(r0.mp);
-    if (!((mp < jb.pb1) && (mp + W > jb.pb0))) continue;
-
-    if (slice < NSL) {
-      const int n = s1 - s0;
-      const int j0 = s0 + (n * slice) / NSL, j1 = s0 + (n * (slice + 1)) / NSL;
-      bool ok[PPL];
-#pragma unroll
-      for (int k = 0; k < PPL; ++k)
-        ok[k] = (pp[k] < W) && (mp + pp[k] >= jb.pb0) && (mp + pp[k] < jb.pb1);
-      // (re, im) accumulators; in FP32 updated with Blackwell's packed
-      // two-lane FMA (one instruction per complex cell)
-      C acc[PPL][W];
-#pragma unroll
-      for (int k = 0; k < PPL; ++k)
-#pragma unroll
-        for (int c = 0; c < W; ++c) acc[k][c].x = acc[k][c].y = R(0);
-      uint32_t cur = 0xffffffffu;
-      int bb0 = 1 << 30, bb1 = -1, bb2 = 1 << 30, bb3 = -1;
-      // the lane's kernel-row indices and tile offsets, fixed for the chunk
-      int kwi[PPL], kui[PPL], coff[PPL];
-#pragma unroll
-      for (int k = 0; k < PPL; ++k) {
-        kwi[k] = 2 * W + (ok[k] ? pp[k] : 0);
-        kui[k] = ok[k] ? cu[k] : 0;
-        coff[k] = pp[k] * tl.PS + cu[k] * tl.RS;
-      }
-      // When every warp works on the same records (SPLIT), the warps reach
-      // each commit together, and for one origin every tile cell belongs to
-      // one lane: a barrier before the commit orders it after the previous
-      // origin's, and the commit is a plain read-modify-write (FP64 shared
-      // atomics cost a quarter of the spread).  Otherwise warps of other
-      // slices may commit to the same cells at any time: shared atomics.
-      auto commit = [&]() {
-        if (cur >= kSkip) return;  // nothing accumulated, or skipped records only (uniform)
-        if constexpr (SPLIT) __syncthreads();
-        const int o = int(cur >> 16) * tl.RS + int(cur & 0xffffu);
-#pragma unroll
-        for (int k = 0; k < PPL; ++k) {
-          if (!ok[k]) continue;
-          const int base = coff[k] + o;
-#pragma unroll
-          for (int c = 0; c < W; ++c) {
-            if constexpr (SPLIT) {
-              tre[base + c] += acc[k][c].x;
-              tim[base + c] += acc[k][c].y;
-            } else {
-              atomicAdd(&tre[base + c], acc[k][c].x);
-              atomicAdd(&tim[base + c], acc[k][c].y);
-            }
-            acc[k][c].x = acc[k][c].y = R(0);
-          }
-        }
-      };
-      for (int b0 = j0; b0 < j1; b0 += 32) {
-        const int nb = min(32, j1 - b0);
-        if constexpr (SPLIT) {
-          __syncthreads();  // every warp is done with the previous batch
-          stage_batch_split<R, W, NWARP>(recs, b0, nb, lane, warp, tu, tv, mp, g, kc, kv, vv,
-                                         luvs, a.err, bb0, bb1, bb2, bb3, a.vis_in,
-                                         a.vis_in_double);
-          __syncthreads();
-        } else {
-          stage_batch<R, W>(recs, b0, nb, lane, tu, tv, mp, g, kc, kv, vv, luvs, a.err, bb0, bb1,
-                            bb2, bb3, a.vis_in, a.vis_in_double);
-          __syncwarp();
-        }
-        if (grp == 0) {
-          // the batch's new footprint origins, by a ballot over the staged
-          // records (a skipped record counts as one; a repeated origin in the
-          // list is harmless, its cells being taken by atomic exchange)
-          const uint32_t my = lane < nb ? luvs[lane] : 0u;
-          uint32_t prev = __shfl_up_sync(0xffffffffu, my, 1);
-          if (lane == 0) prev = cur;
-          const unsigned nm = __ballot_sync(0xffffffffu, lane < nb && my != prev && my != kSkip);
-          if (nm) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&sh_norig, __popc(nm));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            const int k = base + __popc(nm & ((1u << lane) - 1u));
-            if (((nm >> lane) & 1u) && k < kMaxOrig) sh_orig[k] = my;
-          }
-        }
-        for (int jj = 0; jj < nb; ++jj) {
-          const uint32_t luv = luvs[jj];
-          if (__any_sync(0xffffffffu, luv != cur)) {  // warp-uniform: luv is one value
-            commit();
-            cur = luv;
-          }
-          const R *kb = kv + jj * KST;
-          R kvv[W];
-          lds_row<W>(kb + W, kvv);
-          const C vx = reinterpret_cast<const C *>(vv)[jj];
-          const R vr = vx.x, vi = vx.y;
-#pragma unroll
-          for (int k = 0; k < PPL; ++k) {
-            const R f = kb[kwi[k]] * kb[kui[k]];
-            C a;
-            a.x = vr * f;
-            a.y = vi * f;
-#pragma unroll
-            for (int c = 0; c < W; ++c) acc[k][c] = cfma_real(a, kvv[c], acc[k][c]);
-          }
-        }
-        __syncwarp();
-      }
-      commit();
-      warp_minmax(bb0, bb1, bb2, bb3);
-      if (lane == 0 && bb1 >= 0) {
-        atomicMin(&sh_bb[0], bb0); atomicMax(&sh_bb[1], bb1);
-        atomicMin(&sh_bb[2], bb2); atomicMax(&sh_bb[3], bb3);
-      }
-    }
-    __syncthreads();
-    // flush the touched cells of the tile to the band grid: footprint by
-    // footprint when few origins were used (a cell shared by two footprints
-    // is taken by atomic exchange, so it is added once), else the bounding box
-    const int lu0 = sh_bb[0], lv0 = sh_bb[2];
-    const int nbu = max(sh_bb[1] + W - lu0, 0), nbv = max(sh_bb[3] + W - lv0, 0);
-    const int ucorner = tu * g.T - g.nsafe, vcorner = tv * g.T - g.nsafe;
-    const int norig = sh_norig;
-    const bool by_list = norig <= kMaxOrig && norig * W * W < nbu * nbv;
-    // one (plane, row) line per warp-iteration, lanes along v (no divisions);
-    // the line's band row is found once, then each cell only wraps v
-    const int nline = by_list ? norig * W * W : W * nbu;
-    const int linelen = by_list ? W : nbv;
-    const JobRegs jr(jb);
-    // bounding-box lines: (plane, row) of line = p nbu + r, stepped without
-    // a division
-    int bp = 0, br = warp;
-    while (!by_list && nbu > 0 && br >= nbu) { br -= nbu; ++bp; }
-    for (int line = warp; line < nline; line += NWARP) {
-      int p, ia, ib0;
-      if (by_list) {
-        const int o = line / (W * W), pr = line - o * W * W;
-        p = pr / W;
-        const uint32_t luv = sh_orig[o];
-        ia = int(luv >> 16) + (pr - p * W);
-        ib0 = int(luv & 0xffffu);
-      } else {
-        p = bp;
-        ia = lu0 + br;
-        ib0 = lv0;
-        br += NWARP;
-        while (br >= nbu) { br -= nbu; ++bp; }
-      }
-      const int plane = mp + p;
-      const int bi = jr.band_row(jr.wrap_u(ucorner + ia));
-      C *const rowp = (plane >= jr.pb0 && plane < jr.pb1 && bi >= 0)
-                          ? reinterpret_cast<C *>(jr.grid) +
-                                (size_t(bi) * jr.P + (plane - jr.pb0)) * size_t(jr.nv)
-                          : nullptr;
-      R *const lre = tre + p * tl.PS + ia * tl.RS;
-      R *const lim = tim + p * tl.PS + ia * tl.RS;
-      for (int c = lane; c < linelen; c += 32) {
-        const int ib = ib0 + c;
-        R xr, xi;
-        if (by_list) {
-          xr = take_zero(&lre[ib]);
-          xi = take_zero(&lim[ib]);
-        } else {
-          xr = lre[ib];
-          xi = lim[ib];
-          lre[ib] = R(0);
-          lim[ib] = R(0);
-        }
-        if (rowp && (xr != R(0) || xi != R(0))) {
-          C *dst = rowp + jr.wrap_v(vcorner + ib);
-          if constexpr (sizeof(R) == 4) {
-            atomicAdd(reinterpret_cast<float2 *>(dst), make_float2(xr, xi));
-          } else {
-            atomicAdd(&dst->x, xr);
-            atomicAdd(&dst->y, xi);
-          }
-        }
-      }
-    }
-  }
-}
 
 // Writes (or, for batch plans, atomically adds) one degridded visibility.
 __device__ __forceinline__ void store_vis(void *out, int dbl, int accumulate, uint32_t idx,
@@ -1068,267 +574,7 @@ __device__ __forceinline__ void store_vis(void *out, int dbl, int accumulate, ui
   }
 }
 
-// ------------------------------------------------------------- k_interp
-//
-// Degridding, the exact transpose of k_spread: the chunk's tile region is
-// staged from the band grid into shared memory, each lane caches its
-// (plane, u-row) x W cells in registers while the footprint origin repeats,
-// and the kernel-weighted sum is reduced across the warp.  With one warp per
-// record and a single plane pass the result is finalised in place
-// (conjugation, conjugate shift phasor and weight); otherwise partial sums
-// go to a per-record accumulator finalised by k_finalize.
-// IG: records whose warp sums are formed together (4 measured fastest, 8
-// close behind, 1 -- a full butterfly per record -- 10% slower overall)
-template <typename R, int W, int PPL, int NWARP, int IG = 4>
-__global__ void __launch_bounds__(NWARP * 32, sizeof(R) == 4 ? 3 : 1)
-k_interp(GridArgs a, DevGeom g, DevKernel<R> kc) {
-  using Rec = typename RecOf<R>::type;
-  using C = typename Cplx<R>::type;
-  constexpr int NG = WarpGroups<W, PPL, NWARP>::NG;
-  constexpr int NSL = WarpGroups<W, PPL, NWARP>::NSL;
-  constexpr bool SPLIT = WarpGroups<W, PPL, NWARP>::SPLIT;
-  constexpr int KST = KStride<R, W>::value;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const TileLayout tl = a.tl;
-  R *tre = reinterpret_cast<R *>(smem_raw);
-  R *tim = tre + W * tl.PS;
-  __shared__ int sh_chunk, sh_bb[4], sh_norig;
-  __shared__ uint32_t sh_orig[kMaxOrig];
-  __shared__ JobGeom sh_job;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int grp = warp % NG, slice = warp / NG;
-  // the warp's own staging area, and the one it reads records from (warp 0's
-  // when the CTA's warps share the staging)
-  unsigned char *wown = smem_raw + size_t(2 * W * tl.PS) * sizeof(R) + warp * WarpStage<R, W>::bytes;
-  unsigned char *wbase = SPLIT ? smem_raw + size_t(2 * W * tl.PS) * sizeof(R) : wown;
-  R *kv = reinterpret_cast<R *>(wbase);
-  R *vv = kv + 32 * KST;
-  uint32_t *luvs = reinterpret_cast<uint32_t *>(vv + 64);
-  const Rec *recs = reinterpret_cast<const Rec *>(a.rec);
-  // finalised in place in a single plane pass, when one warp owns each
-  // record or all warps share every record (SPLIT: warp 0 adds their sums)
-  const bool direct = a.last_pass && a.first_pass && (NG == 1 || SPLIT);
-
-  int pp[PPL], cu[PPL];
-  bool ok[PPL];
-#pragma unroll
-  for (int k = 0; k < PPL; ++k) {
-    const int q = grp * 32 * PPL + lane + 32 * k;
-    pp[k] = q / W;
-    cu[k] = q - pp[k] * W;
-    ok[k] = q < W * W;
-  }
-
-  for (;;) {
-    __syncthreads();
-    if (tid == 0) {
-      sh_chunk = atomicAdd(a.counter, 1);
-      sh_bb[0] = 1 << 30; sh_bb[1] = -1; sh_bb[2] = 1 << 30; sh_bb[3] = -1;
-      sh_norig = 0;
-      if (sh_chunk < *a.nchunks) sh_job = load_job(a, g, sh_chunk);
-    }
-    __syncthreads();
-    const int ch = sh_chunk;
-    if (ch >= *a.nchunks) break;
-    const JobGeom &jb = sh_job;  // read from shared memory where used
-    const int s0 = a.chunk_start[ch];
-    const int s1 = (ch + 1 < *a.nchunks) ? a.chunk_start[ch + 1] : a.nvis;
-    const Rec r0 = recs[s0];
-    const int tu = int(r0.iuv >> 16) / g.T, tv = int(r0.iuv & 0xffffu) / g.T;
-    const int mp = int(r0.mp);
-    if (!((mp < jb.pb1) && (mp + W > jb.pb0))) continue;  // contributes nothing this pass
-    // bounding box and distinct footprint origins of the chunk
-    for (int s = s0 + tid; s < s1; s += blockDim.x) {
-      const uint32_t iuv = recs[s].iuv;
-      const int lu = int(iuv >> 16) - tu * g.T, lv = int(iuv & 0xffffu) - tv * g.T;
-      if (lu < 0 || lu >= g.T || lv < 0 || lv >= g.T) continue;
-      atomicMin(&sh_bb[0], lu); atomicMax(&sh_bb[1], lu);
-      atomicMin(&sh_bb[2], lv); atomicMax(&sh_bb[3], lv);
-      if (s == s0 || recs[s - 1].iuv != iuv) {
-        const int k = atomicAdd(&sh_norig, 1);
-        if (k < kMaxOrig) sh_orig[k] = (uint32_t(lu) << 16) | uint32_t(lv);
-      }
-    }
-    __syncthreads();
-    {
-      // stage the cells the chunk reads: footprint by footprint when few
-      // origins are used (cells shared by footprints are written twice with
-      // the same value), else the bounding box; eight loads in flight
-      const int lu0 = sh_bb[0], lv0 = sh_bb[2];
-      const int nbu = max(sh_bb[1] + W - lu0, 0), nbv = max(sh_bb[3] + W - lv0, 0);
-      const int ucorner = tu * g.T - g.nsafe, vcorner = tv * g.T - g.nsafe;
-      const int norig = sh_norig;
-      const bool by_list = norig <= kMaxOrig && norig * W * W < nbu * nbv;
-      // (plane, row) lines over warps, lanes along v, eight lines in flight
-      const int nline = by_list ? norig * W * W : W * nbu;
-      const int linelen = by_list ? W : nbv;
-      const JobRegs jr(jb);
-      // bounding-box lines: (plane, row) of line = p nbu + r, stepped by
-      // NWARP lines without a division
-      int bp = 0, br = warp;
-      while (!by_list && nbu > 0 && br >= nbu) { br -= nbu; ++bp; }
-      for (int l0 = warp; l0 < nline; l0 += 8 * NWARP) {
-        C val[8];
-        int sidx[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int line = l0 + q * NWARP;
-          const int lp = bp, lr = br;
-          if (!by_list) {
-            br += NWARP;
-            while (br >= nbu) { br -= nbu; ++bp; }
-          }
-          val[q].x = R(0);
-          val[q].y = R(0);
-          sidx[q] = -1;
-          if (line < nline && lane < linelen) {
-            int p, ia, ib;
-            if (by_list) {
-              const int o = line / (W * W), pr = line - o * W * W;
-              p = pr / W;
-              const uint32_t luv = sh_orig[o];
-              ia = int(luv >> 16) + (pr - p * W);
-              ib = int(luv & 0xffffu) + lane;
-            } else {
-              p = lp;
-              ia = lu0 + lr;
-              ib = lv0 + lane;
-            }
-            sidx[q] = p * tl.PS + ia * tl.RS + ib;
-            const int plane = mp + p;
-            if (plane >= jr.pb0 && plane < jr.pb1) {
-              const int bi = jr.band_row(jr.wrap_u(ucorner + ia));
-              if (bi >= 0)
-                val[q] = reinterpret_cast<const C *>(jr.grid)[(size_t(bi) * jr.P + (plane - jr.pb0)) *
-                                                                  size_t(jr.nv) +
-                                                              jr.wrap_v(vcorner + ib)];
-            }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          if (sidx[q] >= 0) {
-            tre[sidx[q]] = val[q].x;
-            tim[sidx[q]] = val[q].y;
-          }
-        }
-      }
-    }
-    __syncthreads();
-    if (slice < NSL) {
-      const int n = s1 - s0;
-      const int j0 = s0 + (n * slice) / NSL, j1 = s0 + (n * (slice + 1)) / NSL;
-      C cl[PPL][W];  // the lane's cells (re, im) at the current origin
-      uint32_t cur = 0xffffffffu;
-      int bb0 = 0, bb1 = 0, bb2 = 0, bb3 = 0;
-      for (int b0 = j0; b0 < j1; b0 += 32) {
-        const int nb = min(32, j1 - b0);
-        if constexpr (SPLIT) {
-          __syncthreads();  // every warp is done with the previous batch
-          stage_batch_split<R, W, NWARP>(recs, b0, nb, lane, warp, tu, tv, mp, g, kc, kv, vv,
-                                         luvs, a.err, bb0, bb1, bb2, bb3, a.vis_in,
-                                         a.vis_in_double);
-          __syncthreads();
-        } else {
-          stage_batch<R, W>(recs, b0, nb, lane, tu, tv, mp, g, kc, kv, vv, luvs, a.err, bb0, bb1,
-                            bb2, bb3, a.vis_in, a.vis_in_double);
-          __syncwarp();
-        }
-        // record sums of the batch, G records at a time (reduce-scatter);
-        // the staged visibility slots of the warp are free here and hold them
-        constexpr int G = IG;
-        constexpr int LG = G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3;
-        R *osum = reinterpret_cast<R *>(wown) + 32 * KST;
-        for (int g0 = 0; g0 < nb; g0 += G) {
-          C part[G];
-#pragma unroll
-          for (int r = 0; r < G; ++r) {
-            part[r].x = part[r].y = R(0);
-            const int jj = g0 + r;
-            if (jj >= nb) continue;
-            const uint32_t luv = luvs[jj];
-            if (luv == kSkip) continue;
-            if (luv != cur) {
-              cur = luv;
-              const int lu = int(luv >> 16), lv = int(luv & 0xffffu);
-#pragma unroll
-              for (int k = 0; k < PPL; ++k) {
-                const int base = (ok[k] ? pp[k] * tl.PS + (lu + cu[k]) * tl.RS : 0) + lv;
-#pragma unroll
-                for (int c = 0; c < W; ++c) {
-                  cl[k][c].x = ok[k] ? tre[base + c] : R(0);
-                  cl[k][c].y = ok[k] ? tim[base + c] : R(0);
-                }
-              }
-            }
-            const R *kb = kv + jj * KST;
-            R kvv[W];
-            lds_row<W>(kb + W, kvv);
-#pragma unroll
-            for (int k = 0; k < PPL; ++k) {
-              C t;
-              t.x = t.y = R(0);
-#pragma unroll
-              for (int c = 0; c < W; ++c) t = cfma_real(cl[k][c], kvv[c], t);
-              const R f = ok[k] ? kb[2 * W + pp[k]] * kb[cu[k]] : R(0);
-              part[r] = cfma_real(t, f, part[r]);
-            }
-          }
-          const C tot = warp_sum_scatter<G>(part, lane);
-          const int ridx = g0 + ((lane >> (5 - LG)) & (G - 1));
-          if ((lane & ((32 >> LG) - 1)) == 0 && ridx < nb) {
-            osum[2 * ridx] = tot.x;
-            osum[2 * ridx + 1] = tot.y;
-          }
-        }
-        __syncwarp();
-        R osr = lane < nb ? osum[2 * lane] : R(0);
-        R osi = lane < nb ? osum[2 * lane + 1] : R(0);
-        if constexpr (SPLIT) {
-          // every warp summed its pairs of the same records: warp 0 adds the
-          // warps' sums from their staging areas (free until the next
-          // batch's barrier), so each record has one writer
-          __syncthreads();
-          if (warp == 0 && lane < nb) {
-            for (int w = 1; w < NWARP; ++w) {
-              const R *os = reinterpret_cast<const R *>(
-                                smem_raw + size_t(2 * W * tl.PS) * sizeof(R) +
-                                size_t(w) * WarpStage<R, W>::bytes) + 32 * KST;
-              osr += os[2 * lane];
-              osi += os[2 * lane + 1];
-            }
-          }
-        }
-        // lanes finalise their own records of the batch together (one
-        // coalesced record load, instead of one lane per record in turn)
-        if ((!SPLIT || warp == 0) && lane < nb && luvs[lane] != kSkip) {
-          const int s = b0 + lane;
-          if (direct) {
-            const Rec rr = recs[s];
-            const uint32_t idx = rr.idx & 0x7fffffffu;
-            const R si = (rr.idx & 0x80000000u) ? -osi : osi;
-            const double orr = double(rr.vr) * double(osr) - double(rr.vi) * double(si);
-            const double oi = double(rr.vr) * double(si) + double(rr.vi) * double(osr);
-            store_vis(a.vis_out, a.vis_double, a.vis_accumulate, idx, orr, oi);
-          } else if constexpr (SPLIT) {  // the record's one writer in this pass
-            C *accp = reinterpret_cast<C *>(a.acc) + s;
-            accp->x += osr;
-            accp->y += osi;
-          } else {
-            C *accp = reinterpret_cast<C *>(a.acc) + s;
-            atomicAdd(&accp->x, osr);
-            atomicAdd(&accp->y, osi);
-          }
-        }
-        __syncwarp();
-      }
-    }
-  }
-}
-
-// Finalises degridded visibilities accumulated over plane passes or warp
-// groups: out[idx] = P * (flip ? conj(acc) : acc) (added into out when
+// Finalises degridded visibilities accumulated over plane passes: out[idx] = P * (flip ? conj(acc) : acc) (added into out when
 // accumulating).
 template <typename R>
 __global__ void k_finalize(int nvis, const void *recv, const void *accv, void *vis_out,

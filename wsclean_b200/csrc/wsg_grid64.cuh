@@ -247,18 +247,17 @@ k_spread64(GridArgs a, DevGeom g, DevKernel<double> kc) {
     moff[i] = row < 2 * W ? 2 * (row >> 1) * PS + (row & 1) : -1;
   }
 
+  // (a chunk of FP64 records takes many times as long as fetching the next one:
+  // nothing is kept in registers for that meanwhile)
   for (;;) {
+    __syncthreads();  // the tile is clean
+    if (tid == 0) fetch_chunk(cs, a, g);
     __syncthreads();
-    if (tid == 0) next_chunk(cs, a, g);
-    __syncthreads();
-    const int ch = cs.chunk;
-    if (ch >= *a.nchunks) break;
-    const int s0 = a.chunk_start[ch];
-    const int s1 = (ch + 1 < *a.nchunks) ? a.chunk_start[ch + 1] : a.nvis;
-    const RecD r0 = recs[s0];
-    const int tu = int(r0.iuv >> 16) / g.T, tv = int(r0.iuv & 0xffffu) / g.T;
-    const int mp = int(r0.mp);
-    if (!((mp < cs.job.pb1) && (mp + W > cs.job.pb0))) continue;
+    if (cs.chunk < 0) break;
+    const int s0 = cs.s0, s1 = cs.s1;
+    const ChunkBin bin = chunk_bin<W>(cs, recs, g.T);
+    const int tu = bin.tu, tv = bin.tv, mp = bin.mp;
+    if (!bin.pass) continue;
 
     double acc[MT][NT][2];
 #pragma unroll
@@ -466,23 +465,21 @@ k_interp64(GridArgs a, DevGeom g, DevKernel<double> kc) {
 
   for (;;) {
     __syncthreads();
-    if (tid == 0) next_chunk(cs, a, g);
+    if (tid == 0) fetch_chunk(cs, a, g);
     __syncthreads();
-    const int ch = cs.chunk;
-    if (ch >= *a.nchunks) break;
-    const int s0 = a.chunk_start[ch];
-    const int s1 = (ch + 1 < *a.nchunks) ? a.chunk_start[ch + 1] : a.nvis;
-    const RecD r0 = recs[s0];
-    const int tu = int(r0.iuv >> 16) / g.T, tv = int(r0.iuv & 0xffffu) / g.T;
-    const int mp = int(r0.mp);
-    if (!((mp < cs.job.pb1) && (mp + W > cs.job.pb0))) continue;  // nothing in this pass
+    if (cs.chunk < 0) break;
+    const int s0 = cs.s0, s1 = cs.s1;
+    const ChunkBin bin = chunk_bin<W>(cs, recs, g.T);
+    const int tu = bin.tu, tv = bin.tv, mp = bin.mp;
+    if (!bin.pass) continue;  // nothing in this pass
     scan_origins(cs, recs, s0, s1, tu, tv, g.T, tid, NWARP * 32);
     __syncthreads();
     {
       const TileLines tln = tile_lines<W>(cs.bb, cs.norig, cs.orig, lane, NWARP);
-      tile_stage<W, double2>(RS, PS, tln, cs.job, mp, tu * g.T - g.nsafe, tv * g.T - g.nsafe, warp,
-                             lane, NWARP, [&](int at, double2 v) { tile[at] = v; });
+      tile_stage<W, double2>(tile, RS, PS, tln, cs.job, mp, tu * g.T - g.nsafe, tv * g.T - g.nsafe,
+                             warp, lane, NWARP);
     }
+    copies_done();
     __syncthreads();
 
     double cell[MT][KT];

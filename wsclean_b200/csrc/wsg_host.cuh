@@ -102,15 +102,6 @@ DevKernel<R> make_kernel(const PolyKernel &pk) {
   return k;
 }
 
-inline TileLayout make_layout(int T, int W) {
-  TileLayout tl;
-  tl.S = T + W - 1;
-  tl.RS = tl.S | 1;  // odd row stride
-  int ps = tl.S * tl.RS;
-  tl.PS = ps + ((8 - (ps % 32)) + 32) % 32;  // plane stride = 8 mod 32
-  return tl;
-}
-
 // Before the transposed u transform fills the band grid: it writes every
 // band row of the ny image columns (v indices [nv - ny/2, nv) and
 // [0, ny/2)), so only the nv - ny columns between them need clearing.
@@ -222,25 +213,9 @@ std::vector<double> col_twiddle_table(size_t M, size_t nu, size_t K);
 //
 // Defined in wsg_launch.cu for R = float and double.
 
-// Records staged per sub-batch by the spread / interpolation kernels.
-template <typename R>
-constexpr int grid_sb() {
-  return sizeof(R) == 4 ? 256 : 64;
-}
-// Shared memory of a spread / interpolation CTA for this tile layout.
-template <typename R>
-size_t grid_smem_bytes(const TileLayout &tl, int W, bool spread);
-// Warps that share one record.
-template <typename R>
-int grid_groups(int W);
-// Whether the interpolation of one plane pass needs the per-record
-// accumulator (and k_finalize): when a record is shared by some but not
-// all of a CTA's warps (all warps sharing it add their sums in the kernel).
-template <typename R>
-bool grid_needs_acc(int W);
 // One persistent spread (or interpolation) launch over the chunks.
 template <typename R>
-void grid_dispatch(int W, bool spread, int nsm, size_t smem, cudaStream_t st, const GridArgs &a,
+void grid_dispatch(int W, bool spread, int nsm, cudaStream_t st, const GridArgs &a,
                    const DevGeom &g, const DevKernel<R> &kc);
 // The pruned u transform of npl planes (bwd: band to image columns).  err:
 // the device error word (bit 2: a staged copy did not complete), or nullptr

@@ -187,6 +187,13 @@ constexpr int grid64_interp_stride(int W) { return grid64_pad4(3 * W); }
 // Supports whose records a single warp of the interpolation handles.
 constexpr int kSolo64 = 8;
 
+// The FP32 kernels (wsg_grid32.cuh): warps a CTA, floats a staged record takes
+// (4 mod 8).
+constexpr int kGrid32Warps = 8;
+constexpr int grid32_stride(int W) {
+  return 3 * ((W + 3) & ~3) + 2 + (4 - (3 * ((W + 3) & ~3) + 2) % 8 + 8) % 8;
+}
+
 // Shared memory of a spread / interpolation CTA for tile T and support W
 // (the limit leaves 1 KB to the kernels' static variables).
 constexpr size_t kMaxSmemPerBlock = 226 * 1024;

@@ -2,6 +2,7 @@
 // support W), the pruned u transforms (over log2 M, with their staged
 // forms) and the w-screens: the one translation unit that compiles them.
 
+#include "wsg_grid32.cuh"
 #include "wsg_grid64.cuh"
 #include "wsg_host.cuh"
 
@@ -9,102 +10,54 @@ namespace wsg {
 
 namespace {
 
-// Kernel template dispatch over the support W.
+// Spread / interpolation kernels, dispatched over the support W: one
+// persistent launch of as many CTAs as are resident.
 template <typename R>
 struct GridKernels {
-  static constexpr int NWARP = 8;
-  static constexpr int SB = sizeof(R) == 4 ? 256 : 64;
   template <int W>
-  static constexpr int ppl() {
-    return (sizeof(R) == 4 && W * W > 32) ? 2 : 1;
-  }
-  static size_t smem_bytes(const TileLayout &tl, int W, bool spread) {
-    const size_t kst = sizeof(R) == 4 ? ((3 * size_t(W) + 3) & ~size_t(3))
-                                      : ((3 * size_t(W) + 1) & ~size_t(1));
-    const size_t stage = sizeof(R) * (32 * kst + 64) + 128;  // WarpStage<R, W>::bytes
-    size_t tile = ((sizeof(R) * 2 * size_t(W) * tl.PS) + 15) & ~size_t(15);
-    (void)spread;
-    if (sizeof(R) == 8) return tile_smem_bytes(tl.S - W + 1, W, false);
-    const size_t b = tile + size_t(NWARP) * stage;
-    require(b == tile_smem_bytes(tl.S - W + 1, W, sizeof(R) == 4) && b <= kMaxSmemPerBlock,
-            "internal: spread tile exceeds shared memory");
-    return b;
-  }
-  // warps that share one record (more than one when a lane's share of the
-  // W x W (plane, u-row) pairs would exceed PPL)
-  static int groups(int W) {  // WarpGroups<W, ppl, NWARP>::NG
-    const int ppl = (sizeof(R) == 4 && W * W > 32) ? 2 : 1;
-    const int ng = (W * W + 32 * ppl - 1) / (32 * ppl);
-    return ng > NWARP / 2 ? NWARP : ng;
-  }
-  template <int W>
-  static void run(bool spread, dim3 grid, size_t smem, cudaStream_t st, const GridArgs &a,
-                  const DevGeom &g, const DevKernel<R> &kc) {
-    constexpr int P = ppl<W>();
+  static void run(bool spread, int nsm, cudaStream_t st, const GridArgs &a, const DevGeom &g,
+                  const DevKernel<R> &kc) {
+    using Fn = void (*)(GridArgs, DevGeom, DevKernel<R>);
+    Fn fn;
+    int threads;
     if constexpr (sizeof(R) == 8) {
-      auto fn = spread ? k_spread64<W> : k_interp64<W>;
-      smem_attr(fn, smem);
-      fn<<<grid, 32 * (spread ? Cfg64<W>::WARPS : Cfg64<W>::IWARPS), smem, st>>>(a, g, kc);
-    } else if (spread) {
-      auto fn = k_spread<R, W, P, NWARP>;
-      smem_attr(fn, smem);
-      fn<<<grid, NWARP * 32, smem, st>>>(a, g, kc);
+      fn = spread ? k_spread64<W> : k_interp64<W>;
+      threads = 32 * (spread ? Cfg64<W>::WARPS : Cfg64<W>::IWARPS);
     } else {
-      auto fn = k_interp<R, W, P, NWARP>;
-      smem_attr(fn, smem);
-      fn<<<grid, NWARP * 32, smem, st>>>(a, g, kc);
+      fn = spread ? k_spread32<W> : k_interp32<W>;
+      threads = 32 * kWarps32;
     }
-    cuda_check(cudaGetLastError(), spread ? "k_spread launch" : "k_interp launch");
+    const size_t smem = tile_smem_bytes(g.T, W, sizeof(R) == 4);
+    require(smem <= kMaxSmemPerBlock, "internal: spread tile exceeds shared memory");
+    smem_attr(fn, smem);
+    fn<<<nsm * occupancy(reinterpret_cast<const void *>(fn), threads, smem), threads, smem, st>>>(
+        a, g, kc);
+    cuda_check(cudaGetLastError(), spread ? "spread launch" : "interpolation launch");
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
   }
-  template <int W>
-  static int occupancy(bool spread, size_t smem) {
-    // cached: the query is a driver call, and plans enqueue launches while
-    // a stream is being captured into a graph
+  // Resident CTAs an SM, cached: the query is a driver call, and plans enqueue
+  // launches while a stream is being captured into a graph.
+  static int occupancy(const void *fn, int threads, size_t smem) {
     static std::mutex mu;
-    static std::map<std::tuple<int, size_t, int>, int> memo;
+    static std::map<std::tuple<const void *, size_t, int>, int> memo;
     int dev = 0;
     cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    const auto key = std::make_tuple(int(spread), smem, dev);
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      auto it = memo.find(key);
-      if (it != memo.end()) return it->second;
-    }
-    constexpr int P = ppl<W>();
-    int nb = 0;
-    if constexpr (sizeof(R) == 8)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spread ? k_spread64<W> : k_interp64<W>,
-                                                    32 * (spread ? Cfg64<W>::WARPS : Cfg64<W>::IWARPS),
-                                                    smem);
-    else if (spread)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_spread<R, W, P, NWARP>, NWARP * 32, smem);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_interp<R, W, P, NWARP>, NWARP * 32, smem);
-    nb = std::max(nb, 1);
+    const auto key = std::make_tuple(fn, smem, dev);
     std::lock_guard<std::mutex> lk(mu);
-    memo[key] = nb;
-    return nb;
+    auto it = memo.find(key);
+    if (it != memo.end()) return it->second;
+    int nb = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem);
+    return memo[key] = std::max(nb, 1);
   }
-  static void dispatch(int W, bool spread, int nsm, size_t smem, cudaStream_t st, const GridArgs &a,
+  static void dispatch(int W, bool spread, int nsm, cudaStream_t st, const GridArgs &a,
                        const DevGeom &g, const DevKernel<R> &kc) {
     auto go = [&](auto wc) {
       constexpr int WW = decltype(wc)::value;
-      if constexpr (sizeof(R) == 4 && WW > 8) {
+      if constexpr (sizeof(R) == 4 && WW > 8)
         throw std::runtime_error("support too large for mixed precision");
-      } else {
-        // set the smem attribute before asking for the occupancy
-        constexpr int P = ppl<WW>();
-        if constexpr (sizeof(R) == 8)
-          smem_attr(spread ? k_spread64<WW> : k_interp64<WW>, smem);
-        else if (spread)
-          smem_attr(k_spread<R, WW, P, NWARP>, smem);
-        else
-          smem_attr(k_interp<R, WW, P, NWARP>, smem);
-        int occ = occupancy<WW>(spread, smem);
-        dim3 grid(nsm * occ);
-        run<WW>(spread, grid, smem, st, a, g, kc);
-      }
+      else
+        run<WW>(spread, nsm, st, a, g, kc);
     };
     switch (W) {
       case 4: go(std::integral_constant<int, 4>{}); break;
@@ -347,24 +300,9 @@ struct ColKernels {
 }  // namespace
 
 template <typename R>
-size_t grid_smem_bytes(const TileLayout &tl, int W, bool spread) {
-  return GridKernels<R>::smem_bytes(tl, W, spread);
-}
-template <typename R>
-int grid_groups(int W) {
-  return GridKernels<R>::groups(W);
-}
-template <typename R>
-bool grid_needs_acc(int W) {
-  if (sizeof(R) == 8) return false;  // (one writer a record and pass)
-  const int ng = GridKernels<R>::groups(W);
-  return ng > 1 && ng < GridKernels<R>::NWARP;
-}
-template <typename R>
-void grid_dispatch(int W, bool spread, int nsm, size_t smem, cudaStream_t st, const GridArgs &a,
+void grid_dispatch(int W, bool spread, int nsm, cudaStream_t st, const GridArgs &a,
                    const DevGeom &g, const DevKernel<R> &kc) {
-  static_assert(GridKernels<R>::SB == grid_sb<R>(), "sub-batch size");
-  GridKernels<R>::dispatch(W, spread, nsm, smem, st, a, g, kc);
+  GridKernels<R>::dispatch(W, spread, nsm, st, a, g, kc);
 }
 template <typename R>
 void col_run(int logM, bool bwd, const ColArgs &a, int npl, cudaStream_t st, int *err) {
@@ -401,10 +339,7 @@ void launch_screen_put_grid(dim3 grid, cudaStream_t st, const ScreenArgs &s, con
 }
 
 #define WSG_LAUNCHERS(R)                                                                     \
-  template size_t grid_smem_bytes<R>(const TileLayout &, int, bool);                         \
-  template int grid_groups<R>(int);                                                          \
-  template bool grid_needs_acc<R>(int);                                                      \
-  template void grid_dispatch<R>(int, bool, int, size_t, cudaStream_t, const GridArgs &,     \
+  template void grid_dispatch<R>(int, bool, int, cudaStream_t, const GridArgs &,             \
                                  const DevGeom &, const DevKernel<R> &);                     \
   template void col_run<R>(int, bool, const ColArgs &, int, cudaStream_t, int *);            \
   template void launch_screen_add<R>(dim3, cudaStream_t, const ScreenArgs &, const void *,  \

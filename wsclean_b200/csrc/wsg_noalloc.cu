@@ -309,8 +309,6 @@ void ms2dirty_noalloc(const wsg_args &a, const void *vis, void *dirty, cudaStrea
     char *band = reinterpret_cast<char *>(ar.take(gp.band_rows * P * gp.nv * 8));
     char *H = reinterpret_cast<char *>(ar.take(P * gp.ny * gp.hrow() * 8));
     const DevKernel<float> kc = make_kernel<float>(gp.poly);
-    const TileLayout tl = make_layout(gp.T, gp.kernel.W);
-    const size_t smem = grid_smem_bytes<float>(tl, gp.kernel.W, true);
     GridArgs ga{};
     ga.err = d_err;
     ga.rec = rec;
@@ -320,8 +318,6 @@ void ms2dirty_noalloc(const wsg_args &a, const void *vis, void *dirty, cudaStrea
     ga.nvis = int(gp.nvis);
     ga.grid = band;
     ga.P = int(P);
-    ga.tl = tl;
-    ga.sb = grid_sb<float>();
     const ColArgs ca = make_col(gp, P, d_tw, band, H);
     for (size_t pb0 = 0; pb0 < gp.nplanes; pb0 += P) {
       const size_t npl = std::min(P, gp.nplanes - pb0);
@@ -329,7 +325,7 @@ void ms2dirty_noalloc(const wsg_args &a, const void *vis, void *dirty, cudaStrea
       cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), stream), "counter clear");
       ga.pb0 = int(pb0);
       ga.pb1 = int(pb0 + npl);
-      grid_dispatch<float>(gp.kernel.W, true, nsm, smem, stream, ga, g, kc);
+      grid_dispatch<float>(gp.kernel.W, true, nsm, stream, ga, g, kc);
       row_fft_f(logMv, band, (long long)(gp.band_rows * P), d_twv, +1, stream);
       col_run<float>(gp.logM, true, ca, int(npl), stream, d_err);
       ScreenArgs sa = make_screen(gp, d_cf, cc, P);

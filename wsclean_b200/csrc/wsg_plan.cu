@@ -56,7 +56,7 @@ Plan::~Plan() {
   for (auto &j : jobs_)
     for (cufftHandle h : {j.fft, j.gfft})
       if (h) cufftDestroy(h);
-  for (DevBuf *b : {&rec_, &chunks_, &chunk_job_, &jobgeom_, &band_, &H_, &img_, &cf_, &tw_, &acc_,
+  for (DevBuf *b : {&rec_, &chunks_, &chunk_job_, &jobgeom_, &band_, &H_, &img_, &cf_, &tw_,
                     &small_, &fftwork_})
     b->release();
 }
@@ -254,8 +254,6 @@ void Plan::build(const std::vector<wsg_job> &js) {
   CK(cudaMemcpyAsync(cf_.p, cf_host.data(), cf_host.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   tw_.ensure(std::max<size_t>(tw_host.size(), 1));
   CK(cudaMemcpyAsync(tw_.p, tw_host.data(), tw_host.size(), cudaMemcpyHostToDevice, st));
-  need_acc_ = grid_needs_acc<R>(W_);
-  if (need_acc_) acc_.ensure(nrec_ * cs);
   CK(cudaStreamSynchronize(st));
 }
 
@@ -268,16 +266,12 @@ void Plan::enqueue_grid(const void *vis, void *const *dirty, int accumulate) {
   int *d_err = d_nch + 2;
   CK(cudaMemsetAsync(band_.p, 0, band_total_, st));
   CK(cudaMemsetAsync(counter, 0, sizeof(int), st));  // (the error word stays until read)
-  const TileLayout tl = make_layout(T_, W_);
-  const size_t smem = grid_smem_bytes<R>(tl, W_, true);
   GridArgs ga{};
   ga.rec = rec_.p;
   ga.chunk_start = reinterpret_cast<const int *>(chunks_.p);
   ga.nchunks = d_nch;
   ga.counter = counter;
   ga.nvis = int(nrec_);
-  ga.tl = tl;
-  ga.sb = grid_sb<R>();
   ga.err = d_err;
   ga.jobs = reinterpret_cast<const JobGeom *>(jobgeom_.p);
   ga.chunk_job = reinterpret_cast<const int *>(chunk_job_.p);
@@ -287,7 +281,7 @@ void Plan::enqueue_grid(const void *vis, void *const *dirty, int accumulate) {
   std::memcpy(&kc, kernel_.data(), sizeof(kc));
   DevGeom g0;
   std::memcpy(&g0, geom_.data(), sizeof(g0));
-  grid_dispatch<R>(W_, true, cx_.num_sms, smem, st, ga, g0, kc);
+  grid_dispatch<R>(W_, true, cx_.num_sms, st, ga, g0, kc);
   for (size_t j = 0; j < jobs_.size(); ++j) {
     const PlanJob &pj = jobs_[j];
     const GridPlan &gp = pj.gp;
@@ -394,16 +388,12 @@ void Plan::enqueue_degrid(const void *const *dirty, void *vis) {
     g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
   }
   CK(cudaMemsetAsync(counter, 0, sizeof(int), st));  // (the error word stays until read)
-  const TileLayout tl = make_layout(T_, W_);
-  const size_t smem = grid_smem_bytes<R>(tl, W_, false);
   GridArgs ga{};
   ga.rec = rec_.p;
   ga.chunk_start = reinterpret_cast<const int *>(chunks_.p);
   ga.nchunks = d_nch;
   ga.counter = counter;
   ga.nvis = int(nrec_);
-  ga.tl = tl;
-  ga.sb = grid_sb<R>();
   ga.err = d_err;
   ga.jobs = reinterpret_cast<const JobGeom *>(jobgeom_.p);
   ga.chunk_job = reinterpret_cast<const int *>(chunk_job_.p);
@@ -411,19 +401,11 @@ void Plan::enqueue_degrid(const void *const *dirty, void *vis) {
   ga.vis_double = a_.vis_type == WSG_C128;
   ga.vis_accumulate = multi ? 1 : 0;
   ga.first_pass = ga.last_pass = 1;
-  ga.acc = need_acc_ ? acc_.p : nullptr;
-  if (need_acc_) CK(cudaMemsetAsync(acc_.p, 0, nrec_ * cs, st));
   DevKernel<R> kc;
   std::memcpy(&kc, kernel_.data(), sizeof(kc));
   DevGeom g0;
   std::memcpy(&g0, geom_.data(), sizeof(g0));
-  grid_dispatch<R>(W_, false, cx_.num_sms, smem, st, ga, g0, kc);
-  if (need_acc_) {
-    k_finalize<R><<<launch_blocks(nrec_, 256), 256, 0, st>>>(int(nrec_), rec_.p, acc_.p, vis,
-                                                             ga.vis_double, ga.vis_accumulate);
-    cuda_check(cudaGetLastError(), "k_finalize launch");
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  }
+  grid_dispatch<R>(W_, false, cx_.num_sms, st, ga, g0, kc);
 }
 
 void Plan::enqueue(int mode, const void *in, void *const *outs, const void *const *ins, void *out,
@@ -536,7 +518,7 @@ void Plan::stats(size_t job, wsg_stats &o) const {
   o.dw = g.dw;
   o.nshift = g.nshift;
   o.precision = g.fp32 ? WSG_PREC_MIXED : WSG_PREC_FP64;
-  o.device_bytes = rec_.n + chunks_.n + chunk_job_.n + band_.n + H_.n + img_.n + acc_.n + fftwork_.n;
+  o.device_bytes = rec_.n + chunks_.n + chunk_job_.n + band_.n + H_.n + img_.n + fftwork_.n;
   o.kernel_launches = g_kernel_launches.load();
 }
 

@@ -206,8 +206,6 @@ void StreamGridder::add_t(const Staged &s, size_t nrows) {
   GridPlan g = gp_;
   if (!cx_.prepare<R>(ac, s, true, nullptr, g)) return;
   cudaStream_t st = cx_.stream;
-  const TileLayout tl = make_layout(g.T, g.kernel.W);
-  const size_t smem = grid_smem_bytes<R>(tl, g.kernel.W, true);
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 3072);
@@ -227,9 +225,7 @@ void StreamGridder::add_t(const Staged &s, size_t nrows) {
   ga.P = int(g.nplanes);
   ga.pb0 = 0;
   ga.pb1 = int(g.nplanes);
-  ga.tl = tl;
-  ga.sb = grid_sb<R>();
-  grid_dispatch<R>(g.kernel.W, true, cx_.num_sms, smem, st, ga, make_geom(g),
+  grid_dispatch<R>(g.kernel.W, true, cx_.num_sms, st, ga, make_geom(g),
                            make_kernel<R>(g.poly));
 }
 
@@ -504,9 +500,6 @@ void StreamGridder::predict_t(const Staged &s, size_t nrows, void *vis_dev) {
   GridPlan g = gp_;
   if (!cx_.prepare<R>(ac, s, false, vis_dev, g)) return;
   cudaStream_t st = cx_.stream;
-  const size_t cs = 2 * sizeof(R);
-  const TileLayout tl = make_layout(g.T, g.kernel.W);
-  const size_t smem = grid_smem_bytes<R>(tl, g.kernel.W, false);
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 3072);
@@ -523,21 +516,11 @@ void StreamGridder::predict_t(const Staged &s, size_t nrows, void *vis_dev) {
   ga.P = int(g.nplanes);
   ga.pb0 = 0;
   ga.pb1 = int(g.nplanes);
-  ga.tl = tl;
-  ga.sb = grid_sb<R>();
   ga.vis_out = vis_dev;
   ga.vis_double = a_.vis_type == WSG_C128;
   ga.first_pass = ga.last_pass = 1;
-  const bool need_acc = grid_needs_acc<R>(g.kernel.W);
-  ga.acc = need_acc ? cx_.b_acc.ensure(g.nvis * cs) : nullptr;
-  if (need_acc) CK(cudaMemsetAsync(ga.acc, 0, g.nvis * cs, st));
-  grid_dispatch<R>(g.kernel.W, false, cx_.num_sms, smem, st, ga, make_geom(g),
+  grid_dispatch<R>(g.kernel.W, false, cx_.num_sms, st, ga, make_geom(g),
                            make_kernel<R>(g.poly));
-  if (need_acc) {
-    k_finalize<R><<<launch_blocks(g.nvis, 256), 256, 0, st>>>(int(g.nvis), cx_.b_rec.p, ga.acc,
-                                                             vis_dev, ga.vis_double, 0);
-    cuda_check(cudaGetLastError(), "k_finalize launch");
-  }
 }
 
 void StreamGridder::predict(size_t nrows, const double *uvw, void *vis, const void *wgt,

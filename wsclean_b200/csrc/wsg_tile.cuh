@@ -93,6 +93,16 @@ __device__ __forceinline__ float2 take_cell(float2 *p) {
   const unsigned long long v = exch64(p, 0ull);
   return make_float2(__uint_as_float(uint32_t(v)), __uint_as_float(uint32_t(v >> 32)));
 }
+// (put's counterpart for a cell, and whether anything came back)
+__device__ __forceinline__ float2 put_cell(float2 *p, float2 x) {
+  const unsigned long long v =
+      exch64(p, (unsigned long long)__float_as_uint(x.x) |
+                    ((unsigned long long)__float_as_uint(x.y) << 32));
+  return make_float2(__uint_as_float(uint32_t(v)), __uint_as_float(uint32_t(v >> 32)));
+}
+__device__ __forceinline__ bool cell_set(float2 x) {
+  return (__float_as_uint(x.x) | __float_as_uint(x.y)) != 0u;
+}
 __device__ __forceinline__ double2 take_cell(double2 *p) {
   return make_double2(take(&p->x), take(&p->y));
 }
@@ -115,28 +125,51 @@ __device__ __forceinline__ void tile_flush(C *tile, int RS, int PS, const TileLi
     if (lane < t.gsz && l0 + lane < t.nline)
       row = tile_line<W, C>(t, jr, l0 + lane, mp, ucorner, vcorner, RS, PS, where);
     const int n = min(t.gsz, t.nline - l0);
-    for (int i = 0; i < n; i += t.lpi) {
-      const int src = min(i + t.sub, 31);
-      C *const rp = reinterpret_cast<C *>(shfl_ptr(row, src));
-      const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
-      if (t.act && i + t.sub < n) {
-        const C x = take_cell(&tile[(wh & 0xffffu) + t.col]);
-        if (rp && (x.x != 0 || x.y != 0)) {
+    // iterations whose exchanges are in flight together (the FP64 kernels have
+    // no registers to spare)
+    constexpr int U = sizeof(C) == 8 ? 4 : 1;
+    for (int i0 = 0; i0 < n; i0 += U * t.lpi) {
+      C x[U], *dst[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const int i = i0 + q * t.lpi, src = min(i + t.sub, 31);
+        C *const rp = reinterpret_cast<C *>(shfl_ptr(row, src));
+        const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
+        dst[q] = nullptr;
+        if (t.act && i + t.sub < n) {
+          x[q] = take_cell(&tile[(wh & 0xffffu) + t.col]);
           int v = int(wh >> 16) + t.col;
           v -= v >= jr.nv ? jr.nv : 0;
-          red_cell(rp + v, x);
+          if (rp) dst[q] = rp + v;
         }
       }
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+        if (dst[q] && (x[q].x != 0 || x[q].y != 0)) red_cell(dst[q], x[q]);
     }
   }
 }
 
-// Reads the touched cells from the band grid, eight lines in flight; store
-// (tile offset, value) puts one cell into the tile.
-template <int W, typename C, typename Store>
-__device__ __forceinline__ void tile_stage(int RS, int PS, const TileLines &t, const JobGeom &jb,
-                                           int mp, int ucorner, int vcorner, int warp, int lane,
-                                           int nwarp, Store &&store) {
+// One cell from global to shared memory without a register in between (zero
+// when src is null; size 8 or 16 bytes).
+template <typename C>
+__device__ __forceinline__ void copy_cell(C *dst, const C *src, const void *any) {
+  const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+  const void *p = src ? static_cast<const void *>(src) : any;
+  const int n = src ? int(sizeof(C)) : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(__cvta_generic_to_global(p)),
+               "n"(sizeof(C)), "r"(n)
+               : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Copies the touched cells from the band grid into the tile, asynchronously
+// (copies_done and a barrier end it): all of a warp's cells are in flight
+// together.
+template <int W, typename C>
+__device__ __forceinline__ void tile_stage(C *tile, int RS, int PS, const TileLines &t,
+                                           const JobGeom &jb, int mp, int ucorner, int vcorner,
+                                           int warp, int lane, int nwarp) {
   const JobRegs jr(jb);
   for (int l0 = warp * t.gsz; l0 < t.nline; l0 += nwarp * t.gsz) {
     uint32_t where = 0;
@@ -144,46 +177,79 @@ __device__ __forceinline__ void tile_stage(int RS, int PS, const TileLines &t, c
     if (lane < t.gsz && l0 + lane < t.nline)
       row = tile_line<W, C>(t, jr, l0 + lane, mp, ucorner, vcorner, RS, PS, where);
     const int n = min(t.gsz, t.nline - l0);
-    for (int i0 = 0; i0 < n; i0 += 8 * t.lpi) {
-      C val[8];
-      int at[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int i = i0 + q * t.lpi, src = min(i + t.sub, 31);
-        const C *const rp = reinterpret_cast<const C *>(shfl_ptr(row, src));
-        const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
-        val[q].x = val[q].y = 0;
-        at[q] = -1;
-        if (t.act && i + t.sub < n) {
-          at[q] = int(wh & 0xffffu) + t.col;
-          if (rp) {
-            int v = int(wh >> 16) + t.col;
-            v -= v >= jr.nv ? jr.nv : 0;
-            val[q] = rp[v];
-          }
-        }
+    for (int i = 0; i < n; i += t.lpi) {
+      const int src = min(i + t.sub, 31);
+      const C *const rp = reinterpret_cast<const C *>(shfl_ptr(row, src));
+      const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
+      if (t.act && i + t.sub < n) {
+        int v = int(wh >> 16) + t.col;
+        v -= v >= jr.nv ? jr.nv : 0;
+        copy_cell(&tile[(wh & 0xffffu) + t.col], rp ? rp + v : nullptr, jr.grid);
       }
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (at[q] >= 0) store(at[q], val[q]);
     }
   }
 }
 
-// The chunk a CTA works on (read by thread 0 into shared memory).
+// The chunk a CTA works on (filled by thread 0).
 struct ChunkState {
-  int chunk, norig;
+  int chunk, norig;  // chunk < 0: none left
+  int s0, s1;        // its records
   int bb[4];
   uint32_t orig[kMaxOrig];
   JobGeom job;
 };
 
-__device__ __forceinline__ void next_chunk(ChunkState &cs, const GridArgs &a, const DevGeom &g) {
-  cs.chunk = atomicAdd(a.counter, 1);
-  cs.bb[0] = cs.bb[2] = 1 << 30;
-  cs.bb[1] = cs.bb[3] = -1;
-  cs.norig = 0;
-  if (cs.chunk < *a.nchunks) cs.job = load_job(a, g, cs.chunk);
+// Thread 0's fetch of the chunk after the CTA's next one (a CTA keeps three:
+// the one in hand, the next, whose records are loaded early, and the one being
+// fetched), in three parts spread over the work in hand so that none of the
+// dependent loads is waited for.
+struct ChunkFetch {
+  int c, s0, s1;
+  __device__ __forceinline__ void begin(const GridArgs &a) { c = atomicAdd(a.counter, 1); }
+  __device__ __forceinline__ void starts(const GridArgs &a) {
+    const int n = *a.nchunks;
+    if (c >= n) {
+      c = -1;
+      return;
+    }
+    s0 = a.chunk_start[c];
+    s1 = c + 1 < n ? a.chunk_start[c + 1] : a.nvis;
+  }
+  __device__ __forceinline__ void store(ChunkState &cs, const GridArgs &a, const DevGeom &g) const {
+    cs.chunk = c;
+    cs.s0 = s0;
+    cs.s1 = s1;
+    cs.bb[0] = cs.bb[2] = 1 << 30;
+    cs.bb[1] = cs.bb[3] = -1;
+    cs.norig = 0;
+    if (c >= 0) cs.job = load_job(a, g, c);
+  }
+};
+__device__ __forceinline__ void fetch_chunk(ChunkState &cs, const GridArgs &a, const DevGeom &g) {
+  ChunkFetch f;
+  f.begin(a);
+  f.starts(a);
+  f.store(cs, a, g);
+}
+__device__ __forceinline__ void first_chunks(ChunkState *css, const GridArgs &a, const DevGeom &g) {
+  fetch_chunk(css[0], a, g);
+  fetch_chunk(css[1], a, g);
+}
+// A chunk's bin: its first record's tile and plane, and whether it has planes
+// in this pass.
+struct ChunkBin {
+  int tu, tv, mp;
+  bool pass;
+};
+template <int W, typename Rec>
+__device__ __forceinline__ ChunkBin chunk_bin(const ChunkState &cs, const Rec *recs, int T) {
+  const uint32_t iuv = recs[cs.s0].iuv;
+  ChunkBin b;
+  b.mp = int(recs[cs.s0].mp);
+  b.tu = int(iuv >> 16) / T;
+  b.tv = int(iuv & 0xffffu) / T;
+  b.pass = (b.mp < cs.job.pb1) && (b.mp + W > cs.job.pb0);
+  return b;
 }
 
 // Lists a staged batch's new footprint origins (one warp): my is the lane's
