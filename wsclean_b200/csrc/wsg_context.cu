@@ -133,7 +133,8 @@ std::vector<DevBuf *> Context::all_buffers() {
   return {&b_uvw, &b_fovc, &b_vis, &b_wgt, &b_mask, &b_keys_a, &b_keys_b, &b_vals_a,
           &b_vals_b, &b_cub, &b_rec, &b_chunks, &b_small, &b_band, &b_bandf, &b_bandd, &b_H,
           &b_img, &b_img2, &b_acc, &b_fftwork, &b_out, &corr_cache[0].buf, &corr_cache[1].buf,
-          &tw_cache[0].buf, &tw_cache[1].buf, &b_tune, &b_tfovc, &b_mhi, &b_mlo, &b_pad};
+          &tw_cache[0].buf, &tw_cache[1].buf, &tw_cache[2].buf, &tw_cache[3].buf, &tw_cache[4].buf,
+          &tw_cache[5].buf, &b_tune, &b_tfovc, &b_mhi, &b_mlo, &b_pad};
 }
 
 void Context::invalidate_tables() {
@@ -549,18 +550,19 @@ std::vector<double> col_twiddle_table(size_t M, size_t nu, size_t K) {
   return h;
 }
 
-const void *Context::upload_twiddles(const GridPlan &g, bool dbl) {
-  const size_t M = size_t(1) << g.logM;
-  auto key = std::make_tuple(M, g.nu, int(dbl));
+// The tables of a pruned transform of n = K M points.
+const void *Context::upload_twiddles(size_t M, size_t n, size_t K, bool dbl) {
+  auto key = std::make_tuple(M, n, int(dbl));
   const size_t cs = dbl ? 16 : 8;
   for (auto &e : tw_cache)
     if (e.valid && e.key == key) {
       e.used = ++cache_tick;
       return e.buf.p;
     }
-  TwEntry &e = tw_cache[0].used <= tw_cache[1].used ? tw_cache[0] : tw_cache[1];
+  TwEntry &e = *std::min_element(std::begin(tw_cache), std::end(tw_cache),
+                                 [](const TwEntry &a, const TwEntry &b) { return a.used < b.used; });
   {
-    const std::vector<double> h = col_twiddle_table(M, g.nu, size_t(g.K));
+    const std::vector<double> h = col_twiddle_table(M, n, K);
     void *d = e.buf.ensure(h.size() / 2 * cs);
     // stream-ordered (pageable sources are staged before the call returns)
     if (dbl) {
@@ -713,12 +715,15 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
   // the spread writes `band`; the v transform goes out of place to `bandf`,
   // so `band` stays zero outside the columns the spread wrote
   const size_t rowsP = gp.band_rows * P;
-  char *band = reinterpret_cast<char *>(b_band.ensure(rowsP * nv * cs));
+  char *band = reinterpret_cast<char *>(b_band.ensure(rowsP * gp.nvs() * cs));
   // (the whole-grid layout transforms in place and screens the grid itself)
-  char *bandf = gp.ucufft ? nullptr : reinterpret_cast<char *>(b_bandf.ensure(rowsP * nv * cs));
-  char *H = gp.ucufft ? nullptr : reinterpret_cast<char *>(b_H.ensure(P * gp.ny * gp.hrow() * cs));
+  char *bandf =
+      gp.ucufft ? nullptr : reinterpret_cast<char *>(b_bandf.ensure(rowsP * gp.nvt() * cs));
+  char *H = gp.ucufft ? nullptr
+                      : reinterpret_cast<char *>(b_H.ensure(P * gp.ncol() * gp.hrow() * cs));
   ColArgs ca{};
-  if (!gp.ucufft) ca = make_col(gp, P, upload_twiddles(gp, dbl), bandf, H);
+  if (!gp.ucufft) ca = make_col(gp, P, u_tables(gp, dbl), bandf, H);
+  const void *twv = gp.vprune ? v_tables(gp) : nullptr;
   const long Lv = band_v_halfwidth(gp);
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
@@ -739,21 +744,30 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
   for (size_t pb0 = 0; pb0 < gp.nplanes; pb0 += P) {
     const size_t npl = std::min(P, gp.nplanes - pb0);
     CK(cudaEventRecord(ev[2], stream));
-    clear_band(band, rowsP, nv, cs);
+    if (gp.vprune) {
+      CK(cudaMemsetAsync(band, 0, rowsP * gp.nvs() * cs, stream));
+      band_dirty = BandDirty{};
+    } else {
+      clear_band(band, rowsP, nv, cs);
+    }
     CK(cudaMemsetAsync(counter, 0, sizeof(int), stream));
     ga.pb0 = int(pb0);
     ga.pb1 = int(pb0 + npl);
     grid_dispatch<R>(gp.kernel.W, true, num_sms, stream, ga, g, kc);
-    band_dirty = BandDirty{band, rowsP, nv, cs, Lv};
+    if (!gp.vprune) band_dirty = BandDirty{band, rowsP, nv, cs, Lv};
     CK(cudaEventRecord(ev[3], stream));
     if (gp.ucufft) {
       // the whole grid: each plane's 2-D transform in place
       grid_fft(band, gp, P, npl, dir, dbl);
       band_dirty = BandDirty{};  // every entry of `band` written
     } else {
-      // transform along v: every (band row, plane) is a contiguous row of nv
-      cufftHandle h = fft_plan(int(nv), 1, int(nv), 1, int(nv), int(rowsP), dbl);
-      fft_exec(h, band, bandf, dir, dbl);
+      // transform along v: every (band row, plane) is a contiguous row
+      if (gp.vprune) {
+        row_run(gp.logMv, true, make_row(gp, P, npl, twv, band, bandf), num_sms, stream);
+      } else {
+        cufftHandle h = fft_plan(int(nv), 1, int(nv), 1, int(nv), int(rowsP), dbl);
+        fft_exec(h, band, bandf, dir, dbl);
+      }
       // pruned transform along u: band rows of the image columns -> image rows
       col_run<R>(gp.logM, true, ca, int(npl), stream, d_err);
     }
@@ -837,11 +851,15 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
   const size_t rowsP = gp.band_rows * P;
   // (the whole-grid layout: the screen writes the grid `band` itself, which
   // is transformed in place)
-  char *bandi = gp.ucufft ? nullptr : reinterpret_cast<char *>(b_bandd.ensure(rowsP * nv * cs));
-  char *band = reinterpret_cast<char *>(b_bandf.ensure(rowsP * nv * cs));
-  char *H = gp.ucufft ? nullptr : reinterpret_cast<char *>(b_H.ensure(P * gp.ny * gp.hrow() * cs));
+  // (with the pruned v transform, bandi holds the transformed columns only)
+  char *bandi =
+      gp.ucufft ? nullptr : reinterpret_cast<char *>(b_bandd.ensure(rowsP * gp.nvt() * cs));
+  char *band = reinterpret_cast<char *>(b_bandf.ensure(rowsP * gp.nvs() * cs));
+  char *H = gp.ucufft ? nullptr
+                      : reinterpret_cast<char *>(b_H.ensure(P * gp.ncol() * gp.hrow() * cs));
   ColArgs ca{};
-  if (!gp.ucufft) ca = make_col(gp, P, upload_twiddles(gp, dbl), bandi, H);
+  if (!gp.ucufft) ca = make_col(gp, P, u_tables(gp, dbl), bandi, H);
+  const void *twv = gp.vprune ? v_tables(gp) : nullptr;
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
@@ -885,6 +903,10 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
     CK(cudaEventRecord(ev[3], stream));
     if (gp.ucufft) {
       grid_fft(band, gp, P, npl, dir, dbl);  // each plane's 2-D transform in place
+    } else if (gp.vprune) {
+      bandd_zero = BandDirty{};
+      col_run<R>(gp.logM, false, ca, int(npl), stream, d_err);
+      row_run(gp.logMv, false, make_row(gp, P, npl, twv, band, bandi), num_sms, stream);
     } else {
       // pruned transform along u (transposed): image rows -> band rows of the
       // image columns; the other columns of the band grid stay zero

@@ -188,7 +188,13 @@ class Context {
   template <typename R>
   bool prepare(const wsg_args &a, const Staged &s, bool gridding, void *vis_out_dev, GridPlan &gp);
   ChebCorr upload_corrections(const GridPlan &g);
-  const void *upload_twiddles(const GridPlan &g, bool dbl);
+  const void *upload_twiddles(size_t M, size_t n, size_t K, bool dbl);
+  const void *u_tables(const GridPlan &g, bool dbl) {
+    return upload_twiddles(size_t(1) << g.logM, g.nu, size_t(g.K), dbl);
+  }
+  const void *v_tables(const GridPlan &g) {
+    return upload_twiddles(size_t(1) << g.logMv, g.nv, size_t(g.Kv), false);
+  }
   size_t choose_planes(const GridPlan &g, bool gridding);
   cufftHandle fft_plan(int n, int istride, int idist, int ostride, int odist, int batch, bool dbl);
   void fft_exec(cufftHandle h, void *in, void *out, int dir, bool dbl);
@@ -246,7 +252,7 @@ class Context {
     bool valid = false;
   };
   CorrEntry corr_cache[2];
-  TwEntry tw_cache[2];
+  TwEntry tw_cache[6];
   uint64_t cache_tick = 0;
   const double *cf_cur = nullptr;  // the tables the last upload_corrections chose
   void invalidate_tables();
@@ -266,7 +272,7 @@ struct PlanJob {
   size_t rec_off = 0, nrec = 0;
   size_t band_off = 0, band_bytes = 0;  // bytes in the plan's band buffer
   size_t cf_off = 0;        // doubles in the plan's correction buffer
-  size_t tw_off = 0;        // bytes in the plan's twiddle buffer
+  size_t tw_off = 0, twv_off = 0;  // bytes in the plan's twiddle buffer (u, pruned v)
   ChebCorr cc;
   cufftHandle fft = 0;
   cufftHandle gfft = 0;      // the whole-grid layout's plane transform (GridPlan::ucufft)
@@ -300,7 +306,7 @@ class Plan {
   wsg_args a_;
   bool dbl_ = false;
   std::vector<PlanJob> jobs_;
-  DevBuf rec_, chunks_, chunk_job_, jobgeom_, band_, H_, img_, cf_, tw_, small_, fftwork_;
+  DevBuf rec_, chunks_, chunk_job_, jobgeom_, band_, H_, hv_, img_, cf_, tw_, small_, fftwork_;
   size_t nrec_ = 0, band_total_ = 0, max_npix_ = 0;
   int nchunks_ = 0;
   std::vector<unsigned char> kernel_;  // DevKernel<R> bytes
@@ -356,7 +362,7 @@ class StreamGridder {
   template <typename R>
   void finish_t(void *dirty, int accumulate);
   template <typename R>
-  void predict_begin_t(const double *img);
+  void predict_begin_t(const void *img, int in_f32);
   template <typename R>
   void predict_t(const Staged &s, size_t nrows, void *vis_dev);
   Staged stage(Slot &sl, size_t nrows, const double *uvw, const void *vis, const void *wgt,
@@ -389,7 +395,7 @@ class StreamGridder {
   GridPlan gp_;
   bool dbl_ = false;
   int mode_ = 0;  // 0 idle, 1 gridding, 2 predicting
-  DevBuf band_, H_, img_, cf_, tw_, fftwork_, vout_;
+  DevBuf band_, H_, hv_, img_, cf_, tw_, twv_, fftwork_, vout_;
   ChebCorr cc_;
   cufftHandle fft_ = 0;
   cudaStream_t copy_ = nullptr;

@@ -54,6 +54,7 @@ struct DevGeom {
   int wide;                               // 64-bit sort keys
   unsigned long long inactive_key;
   int Lu, band_rows, band_full;
+  int Lv, nvs;   // occupied v columns stored [-Lv, Lv], nvs a row (Lv < 0: all nv)
 };
 
 struct ScanOut {
@@ -470,7 +471,8 @@ struct ChunkStartPred {
 struct JobGeom {
   int nu, nv, Lu, band_rows, band_full;
   int P, pb0, pb1;   // planes in the band layout, planes of this pass [pb0, pb1)
-  void *grid;        // the job's u-band grid [band_rows][P][nv] complex
+  int Lv, nvs;       // as DevGeom
+  void *grid;        // the job's band grid [band_rows][P][nvs] complex
 };
 
 struct GridArgs {
@@ -479,7 +481,7 @@ struct GridArgs {
   const int *nchunks;
   int *counter;
   int nvis;
-  void *grid;        // u-band grid [band_rows][P][nv] complex
+  void *grid;        // band grid [band_rows][P][nvs] complex
   int P;             // planes in the layout
   int pb0, pb1;      // planes of this pass: [pb0, pb1)
   int *err;          // set to 1 if a record falls outside its chunk's tile
@@ -512,6 +514,8 @@ __device__ __forceinline__ JobGeom load_job(const GridArgs &a, const DevGeom &g,
   j.P = a.P;
   j.pb0 = a.pb0;
   j.pb1 = a.pb1;
+  j.Lv = g.Lv;
+  j.nvs = g.nvs;
   j.grid = a.grid;
   return j;
 }
@@ -521,12 +525,12 @@ __device__ __forceinline__ JobGeom load_job(const GridArgs &a, const DevGeom &g,
 // into registers: inside loops that also store to shared memory the compiler
 // would otherwise reload every field for every cell.
 struct JobRegs {
-  int nu, nv, Lu, rows, P, pb0, pb1;
+  int nu, nv, Lu, rows, P, pb0, pb1, Lv, nvs;
   bool full;
   void *grid;
   __device__ __forceinline__ explicit JobRegs(const JobGeom &j)
       : nu(j.nu), nv(j.nv), Lu(j.Lu), rows(j.band_rows), P(j.P), pb0(j.pb0), pb1(j.pb1),
-        full(j.band_full), grid(j.grid) {}
+        Lv(j.Lv), nvs(j.nvs), full(j.band_full), grid(j.grid) {}
   // band row of grid row u (wrapped into [0, nu)), or -1 outside the band
   __device__ __forceinline__ int band_row(int u) const {
     if (full || u <= Lu) return u;
@@ -539,6 +543,20 @@ struct JobRegs {
   __device__ __forceinline__ int wrap_v(int v) const {
     v += (v < 0) ? nv : 0;
     return v - ((v >= nv) ? nv : 0);
+  }
+  // Stored column of v where a tile line starts (the columns after it are
+  // checked by next_col; far outside the band, a column that stays outside
+  // over a line's 32 cells), and of a cell c further on, or -1 outside.
+  __device__ __forceinline__ int first_col(int v) const {
+    v = wrap_v(v);
+    if (Lv < 0) return v;
+    v = (v > nv / 2 ? v - nv : v) + Lv;
+    return min(max(v, -64), nvs);
+  }
+  __device__ __forceinline__ int next_col(int first, int c) const {
+    const int v = first + c;
+    if (Lv < 0) return v - (v >= nv ? nv : 0);
+    return unsigned(v) < unsigned(nvs) ? v : -1;
   }
 };
 
@@ -726,14 +744,16 @@ struct FftStages {
 };
 
 struct ColArgs {
-  int nx, ny, nu, nv;
+  int nx, nu;
+  int ny, nv, joff;     // columns transformed, entries of a band row, and the band
+                        // entry of column 0 (column j is at (joff + j) mod nv)
   int P, npl;           // planes in the band layout, planes in this pass
   int L, band_rows, band_full, K;
   const void *twM;      // per-stage FFT twiddles, M entries
   const void *twB;      // exp(+2 pi i t k2 / nu), [k2][t], K x M/16 entries
   const void *twQ;      // exp(+2 pi i (M/16 q - neg M) k2 / nu), [k2][q][neg], K x 32
-  void *band;           // [band_rows][P][nv] complex
-  void *H;              // [P][ny][K * hseg] complex: u-transformed image columns
+  void *band;           // [band_rows][P][nv] complex, transformed along v
+  void *H;              // [P][ny][K * hseg] complex: u-transformed columns
   int hseg, hm0;        // row layout of H (GridPlan::hseg / hm0)
 };
 
@@ -838,8 +858,12 @@ __device__ __forceinline__ void col_tail(C *cur, C *oth, const C *tw, int t, C (
 // In-place col_tail: the data in buf, each middle stage reading all its
 // inputs before a barrier and writing back in place; the last stage leaves
 // its outputs in o[q] = X[t + TPF q].
-template <typename C, int M, int NS, int TPF, int SIGN>
-__device__ __forceinline__ void col_tail_inplace(C *buf, const C *tw, int t, C (&o)[16]) {
+struct CtaSync {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+template <typename C, int M, int NS, int TPF, int SIGN, typename Sync>
+__device__ __forceinline__ void col_tail_inplace(C *buf, const C *tw, int t, C (&o)[16],
+                                                 const Sync &sync) {
   if constexpr (M / NS > 16) {
     C v[16];
 #pragma unroll
@@ -854,11 +878,11 @@ __device__ __forceinline__ void col_tail_inplace(C *buf, const C *tw, int t, C (
     }
     dft_reg<16>(v, SIGN);
     const int d = (t / NS) * NS * 16 + k;
-    __syncthreads();
+    sync();
 #pragma unroll
     for (int r = 0; r < 16; ++r) buf[fpad(d + r * NS)] = v[r];
-    __syncthreads();
-    col_tail_inplace<C, M, NS * 16, TPF, SIGN>(buf, tw, t, o);
+    sync();
+    col_tail_inplace<C, M, NS * 16, TPF, SIGN>(buf, tw, t, o, sync);
   } else {
     constexpr int RL = M / NS, IT = 16 / RL;
     constexpr int off = TwOffset<NS>::value;
@@ -978,7 +1002,7 @@ k_ucol_bwd(ColArgs a) {
       val[q].y = R(0);
       const int u = slot_u(a, b, M);
       if (jj < a.ny && u < (1 << 29)) {
-        int jx = jj + a.nv - a.ny / 2;
+        int jx = jj + a.joff;
         jx -= (jx >= a.nv) ? a.nv : 0;
         val[q] = band[(size_t(slot_bi(a, u)) * a.P + lp) * a.nv + jx];
       }
@@ -1097,7 +1121,7 @@ __device__ __forceinline__ void tma_issue_item(const ColArgs &a, const CUtensorM
                                                typename Cplx<R>::type *stage, uint64_t *bar,
                                                int lp, int j0) {
   using Cfg = TmaCfg<R, M>;
-  int jx = j0 + a.nv - a.ny / 2;
+  int jx = j0 + a.joff;
   jx -= (jx >= a.nv) ? a.nv : 0;
   const int x = 2 * (lp * a.nv + jx);
   const int n1 = tma_boxes1(a, M, Cfg::BR);
@@ -1112,15 +1136,15 @@ __device__ __forceinline__ void tma_issue_item(const ColArgs &a, const CUtensorM
 // In-place variant of col_fft: v[q] = x[t + TPF q] -> o[q] = X[t + TPF q],
 // every exchange through the one buffer buf, with a barrier between the
 // reads and the writes of each stage.
-template <typename C, int M, int TPF, int SIGN>
-__device__ __forceinline__ void col_fft_inplace(C (&v)[16], C *buf, const C *tw, int t,
-                                                C (&o)[16]) {
+template <typename C, int M, int TPF, int SIGN, typename Sync = CtaSync>
+__device__ __forceinline__ void col_fft_inplace(C (&v)[16], C *buf, const C *tw, int t, C (&o)[16],
+                                                const Sync &sync = Sync()) {
   dft_reg<16>(v, SIGN);
-  __syncthreads();  // earlier readers of buf are done
+  sync();  // earlier readers of buf are done
 #pragma unroll
   for (int r = 0; r < 16; ++r) buf[fpad(16 * t + r)] = v[r];
-  __syncthreads();
-  col_tail_inplace<C, M, 16, TPF, SIGN>(buf, tw, t, o);
+  sync();
+  col_tail_inplace<C, M, 16, TPF, SIGN>(buf, tw, t, o, sync);
 }
 
 // One-column geometries (M = 4096 and 8192 in FP32, where a CTA of M/16
@@ -1160,7 +1184,7 @@ k_ucol_bwd_pair(ColArgs a) {
       val[q].y = R(0);
       const int u = slot_u(a, b, M);
       if (jj < a.ny && u < (1 << 29)) {
-        int jx = jj + a.nv - a.ny / 2;
+        int jx = jj + a.joff;
         jx -= (jx >= a.nv) ? a.nv : 0;
         val[q] = band[(size_t(slot_bi(a, u)) * a.P + lp) * a.nv + jx];
       }
@@ -1280,7 +1304,7 @@ k_ucol_fwd_pair(ColArgs a) {
     const int jj = j0 + c;
     const int u = slot_u(a, b, M);
     if (jj < a.ny && u < (1 << 29)) {
-      int jx = jj + a.nv - a.ny / 2;
+      int jx = jj + a.joff;
       jx -= (jx >= a.nv) ? a.nv : 0;
       band[(size_t(slot_bi(a, u)) * a.P + lp) * a.nv + jx] = buf[c * BL + fpad(b)];
     }
@@ -1388,7 +1412,7 @@ __global__ void __launch_bounds__(ColBig<(1 << LOGM)>::TPF, 1) k_ucol_bwd_big(Co
   const C *twQ = reinterpret_cast<const C *>(a.twQ);
   const C *twg = reinterpret_cast<const C *>(a.twM);
   C *rowp = reinterpret_cast<C *>(a.H) + (size_t(lp) * a.ny + j) * (size_t(a.K) * a.hseg);
-  int jx = j + a.nv - a.ny / 2;
+  int jx = j + a.joff;
   jx -= (jx >= a.nv) ? a.nv : 0;
   // (ordered before its first use by the transform's barriers)
   fill_table<C, ColBig<M>::NTAB, TPF>(tws, twg);
@@ -1431,7 +1455,7 @@ __global__ void __launch_bounds__(ColBig<(1 << LOGM)>::TPF, 1) k_ucol_fwd_big(Co
   const C *twQ = reinterpret_cast<const C *>(a.twQ);
   const C *twg = reinterpret_cast<const C *>(a.twM);
   const C *rowp = reinterpret_cast<const C *>(a.H) + (size_t(lp) * a.ny + j) * (size_t(a.K) * a.hseg);
-  int jx = j + a.nv - a.ny / 2;
+  int jx = j + a.joff;
   jx -= (jx >= a.nv) ? a.nv : 0;
   fill_table<C, ColBig<M>::NTAB, TPF>(tws, twg);
   for (int k2 = 0; k2 < a.K; ++k2) {
@@ -1649,7 +1673,7 @@ k_ucol_fwd(ColArgs a) {
     const int jj = blockIdx.x * NB + c;
     const int u = slot_u(a, b, M);
     if (jj < a.ny && u < (1 << 29)) {
-      int jx = jj + a.nv - a.ny / 2;
+      int jx = jj + a.joff;
       jx -= (jx >= a.nv) ? a.nv : 0;
       band[(size_t(slot_bi(a, u)) * a.P + lp) * a.nv + jx] = bufall[c * 2 * BL + fpad(b)];
     }
@@ -1796,7 +1820,7 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
       const int jj = jb + c;
       const int u = slot_u(a, b, M);
       if (jj < a.ny && u < (1 << 29)) {
-        int jx = jj + a.nv - a.ny / 2;
+        int jx = jj + a.joff;
         jx -= (jx >= a.nv) ? a.nv : 0;
         band[(size_t(slot_bi(a, u)) * a.P + lp) * a.nv + jx] = bufall[c * BL + fpad(b)];
       }
@@ -1999,6 +2023,7 @@ static __global__ void k_wsplit(size_t nrows, int nchan, const double *__restric
 
 struct ScreenArgs {
   int nx, ny, nu, nv;
+  int ncol, Kv, hsegv, hm0v;  // columns of H and their order (screen_col)
   size_t ld;                // row stride of the x-major image (ny, or the full
                             // image's ny for a facet inside a larger image)
   double px, py, x0, y0;
@@ -2045,14 +2070,12 @@ __device__ __forceinline__ void pixel_terms(const ScreenArgs &s, int i, int j,
   q = nm1 + s.nshift;
 }
 
-// Offset in H, [P][ny][K hseg], of pixel (i, j)'s entry -- image row i
-// being entry mm of segment k2 -- in the first plane, and the stride between
-// planes.
-__device__ __forceinline__ size_t screen_h_off(const ScreenArgs &s, int i, int j, int k2, int mm,
+// Offset in H, [P][ncol][K hseg], of entry mm of segment k2 of column j in the
+// first plane, and the stride between planes.
+__device__ __forceinline__ size_t screen_h_off(const ScreenArgs &s, int j, int k2, int mm,
                                                size_t &pstride) {
-  (void)i;
   const size_t hrow = size_t(s.K) * s.hseg;
-  pstride = size_t(s.ny) * hrow;
+  pstride = size_t(s.ncol) * hrow;
   return size_t(j) * hrow + (size_t(k2) * s.hseg + mm);
 }
 
@@ -2077,6 +2100,13 @@ __device__ __forceinline__ int screen_row(const ScreenArgs &s, int k2, int mm) {
   return (mm < s.hseg && unsigned(i) < unsigned(s.nx)) ? i : -1;
 }
 
+// Image column of column c of H, or -1 for a column that holds none.
+__device__ __forceinline__ int screen_col(const ScreenArgs &s, int c) {
+  const int k = c / s.hsegv;
+  const int j = s.Kv * (c - k * s.hsegv + s.hm0v) + k + s.ny / 2;
+  return (c < s.ncol && unsigned(j) < unsigned(s.ny)) ? j : -1;
+}
+
 // ms2dirty: img(i,j) += corr(i,j) * sum_p Re(H[p][j][pos(i)] * exp(-2 pi i w_p q)),
 // FP64 pixel terms, the phases by a recurrence over planes in the grid's
 // precision (screen_phase), FP64 accumulation of the per-block sums.
@@ -2097,11 +2127,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) k_screen_add(Scre
   // FP64 terms are computed
   constexpr int PB = sizeof(R) == 4 ? 16 : 8;
   for (int k = 0; k < 4; ++k) {
-    const int j = j0 + ty + 8 * k;
+    const int c = j0 + ty + 8 * k, j = screen_col(s, c);
     double val = 0;
-    if (i >= 0 && j < s.ny) {
+    if (i >= 0 && j >= 0) {
       size_t pstride;
-      const C *hp = H + screen_h_off(s, i, j, k2, mm0 + tx, pstride);
+      const C *hp = H + screen_h_off(s, c, k2, mm0 + tx, pstride);
       C hb[PB];
 #pragma unroll
       for (int u = 0; u < PB; ++u)
@@ -2150,8 +2180,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 3) k_screen_add(Scre
   }
   __syncthreads();
   for (int k = 0; k < 4; ++k) {
-    const int ii = screen_row(s, k2, mm0 + ty + 8 * k), jj = j0 + tx;
-    if (ii >= 0 && jj < s.ny) {
+    const int ii = screen_row(s, k2, mm0 + ty + 8 * k), jj = screen_col(s, j0 + tx);
+    if (ii >= 0 && jj >= 0) {
       const size_t o = size_t(ii) * s.ld + jj;
       const double x = tile[tx][ty + 8 * k];
       if (out_mode == 0)
@@ -2176,9 +2206,9 @@ __global__ void __launch_bounds__(256) k_screen_put(ScreenArgs s, const void *im
   const int j0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int k = 0; k < 4; ++k) {  // coalesced read along j
-    const int ii = screen_row(s, k2, mm0 + ty + 8 * k), jj = j0 + tx;
+    const int ii = screen_row(s, k2, mm0 + ty + 8 * k), jj = screen_col(s, j0 + tx);
     double x = 0.0;
-    if (ii >= 0 && jj < s.ny) {
+    if (ii >= 0 && jj >= 0) {
       const size_t o = size_t(ii) * s.ld + jj;
       x = in_f32 ? double(reinterpret_cast<const float *>(img)[o])
                  : reinterpret_cast<const double *>(img)[o];
@@ -2188,14 +2218,14 @@ __global__ void __launch_bounds__(256) k_screen_put(ScreenArgs s, const void *im
   __syncthreads();
   const int i = screen_row(s, k2, mm0 + tx);
   for (int k = 0; k < 4; ++k) {
-    const int j = j0 + ty + 8 * k;
-    if (i < 0 || j >= s.ny) continue;
+    const int c = j0 + ty + 8 * k, j = screen_col(s, c);
+    if (i < 0 || j < 0) continue;
     double corr, q;
     bool inside;
     pixel_terms(s, i, j, corr, q, inside);
     const double val = tile[ty + 8 * k][tx] * corr;
     size_t pstride;
-    C *hp = H + screen_h_off(s, i, j, k2, mm0 + tx, pstride);
+    C *hp = H + screen_h_off(s, c, k2, mm0 + tx, pstride);
     if (s.do_w && inside) {
       const double w0 = s.wmin + s.pb0 * s.dw;
       const auto st = screen_phase<R>(s.dw * q);

@@ -29,6 +29,7 @@
 
 #include "wsg_context.h"
 #include "wsg_device.cuh"
+#include "wsg_rows.cuh"
 
 namespace wsg {
 
@@ -83,6 +84,8 @@ inline DevGeom make_geom(const GridPlan &g) {
   d.Lu = int(g.Lu);
   d.band_rows = int(g.band_rows);
   d.band_full = g.band_full;
+  d.Lv = g.vprune ? int(g.Lv) : -1;
+  d.nvs = int(g.nvs());
   return d;
 }
 
@@ -149,6 +152,10 @@ inline ScreenArgs make_screen(const GridPlan &g, const double *d_cf, const ChebC
   ScreenArgs s{};
   s.nx = int(g.nx);
   s.ny = int(g.ny);
+  s.ncol = int(g.ncol());
+  s.Kv = g.vprune ? g.Kv : 1;
+  s.hsegv = int(g.hsegv());
+  s.hm0v = g.vprune ? g.hm0v() : -int(g.ny / 2);
   s.nu = int(g.nu);
   s.nv = int(g.nv);
   s.ld = g.ny;
@@ -177,9 +184,10 @@ inline ScreenArgs make_screen(const GridPlan &g, const double *d_cf, const ChebC
 inline ColArgs make_col(const GridPlan &g, size_t P, const void *tw, void *band, void *H) {
   ColArgs c{};
   c.nx = int(g.nx);
-  c.ny = int(g.ny);
+  c.ny = int(g.ncol());
   c.nu = int(g.nu);
-  c.nv = int(g.nv);
+  c.nv = int(g.nvt());
+  c.joff = g.vprune ? 0 : int(g.nv - g.ny / 2);
   c.P = int(P);
   c.L = int(g.Lu);
   c.band_rows = int(g.band_rows);
@@ -202,7 +210,31 @@ inline ColArgs make_col(const GridPlan &g, size_t P, const void *tw, void *band,
 // by 8 image rows a block.
 inline dim3 screen_grid(const GridPlan &g) {
   if (g.ucufft) return dim3(unsigned((g.ny + 31) / 32), unsigned((g.nx + 7) / 8));
-  return dim3(unsigned(size_t(g.K) * ((g.hseg() + 31) / 32)), unsigned((g.ny + 31) / 32));
+  return dim3(unsigned(size_t(g.K) * ((g.hseg() + 31) / 32)), unsigned((g.ncol() + 31) / 32));
+}
+
+// Arguments of the pruned v transform of npl planes: band and hv at the first
+// of them, P planes in both layouts.
+inline RowArgs make_row(const GridPlan &g, size_t P, size_t npl, const void *tw, void *band,
+                        void *hv) {
+  RowArgs r{};
+  r.band = band;
+  r.hv = hv;
+  r.nrow = (long long)(g.band_rows * npl);
+  r.P = int(P);
+  r.npl = int(npl);
+  r.nvs = int(g.nvs());
+  r.Lv = int(g.Lv);
+  r.ncol = int(g.ncol());
+  r.K = g.Kv;
+  r.hseg = int(g.hsegv());
+  r.hm0 = g.hm0v();
+  r.ny = int(g.ny);
+  const size_t M = size_t(1) << g.logMv;
+  r.twM = tw;
+  r.twB = reinterpret_cast<const char *>(tw) + M * 8;
+  r.twQ = reinterpret_cast<const char *>(tw) + (M + size_t(g.Kv) * (M / 16)) * 8;
+  return r;
 }
 
 // Twiddle tables of the pruned u transform (wsg_context.cu).
@@ -222,6 +254,8 @@ void grid_dispatch(int W, bool spread, int nsm, cudaStream_t st, const GridArgs 
 // to stay with the plain loads.
 template <typename R>
 void col_run(int logM, bool bwd, const ColArgs &a, int npl, cudaStream_t st, int *err = nullptr);
+// The pruned v transform (GridPlan::vprune; bwd: band rows to columns).
+void row_run(int logM, bool bwd, const RowArgs &a, int nsm, cudaStream_t st);
 // The w-screens (grid: screen_grid).
 template <typename R>
 void launch_screen_add(dim3 grid, cudaStream_t st, const ScreenArgs &s, const void *H,

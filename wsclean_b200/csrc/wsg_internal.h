@@ -128,6 +128,26 @@ struct GridPlan {
   // column, nu entries) the w-screens read and write in place of the
   // segmented rows below.
   bool ucufft = false;
+  // Mixed precision, when the occupied v columns fit a pruned transform too:
+  // nv = Kv * 2^logMv with 2^logMv >= 2 Lv + 1.  The band grid then stores the
+  // columns v = -Lv .. Lv only, and the rows transformed along v hold the
+  // image columns in Kv segments (as the u-transformed rows below).  Otherwise
+  // (vprune false) the band grid holds all nv columns and the v transform is
+  // the library's.
+  bool vprune = false;
+  size_t Lv = 0;
+  int logMv = 0, Kv = 1;
+  // entries of a band grid row, and of a row transformed along v
+  size_t nvs() const { return vprune ? (2 * Lv + 2) & ~size_t(1) : nv; }
+  int hm0v() const { return -int((ny / 2 + Kv - 1) / Kv); }
+  size_t hsegv() const {
+    if (!vprune || Kv == 1) return ny;
+    const size_t nm = size_t(int((ny - 1 - ny / 2) / Kv) - hm0v() + 1);
+    return (nm + 31) & ~size_t(31);
+  }
+  size_t nvt() const { return vprune ? ncol() : nv; }
+  // transformed columns (image columns, and the padding of their segments)
+  size_t ncol() const { return vprune ? size_t(Kv) * hsegv() : ny; }
   // Layout of one u-transformed image row (the array between the u
   // transform and the w-screen): pixel row i, at s = i - nx/2 = K m + k2
   // (0 <= k2 < K), is written by the k2-th pruned FFT as its output m.  The

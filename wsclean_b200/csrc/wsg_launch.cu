@@ -10,6 +10,22 @@ namespace wsg {
 
 namespace {
 
+// Resident CTAs an SM, cached: the query is a driver call, and plans enqueue
+// launches while a stream is being captured into a graph.
+int resident_ctas(const void *fn, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void *, size_t, int>, int> memo;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  const auto key = std::make_tuple(fn, smem, dev);
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = memo.find(key);
+  if (it != memo.end()) return it->second;
+  int nb = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem);
+  return memo[key] = std::max(nb, 1);
+}
+
 // Spread / interpolation kernels, dispatched over the support W: one
 // persistent launch of as many CTAs as are resident.
 template <typename R>
@@ -30,25 +46,10 @@ struct GridKernels {
     const size_t smem = tile_smem_bytes(g.T, W, sizeof(R) == 4);
     require(smem <= kMaxSmemPerBlock, "internal: spread tile exceeds shared memory");
     smem_attr(fn, smem);
-    fn<<<nsm * occupancy(reinterpret_cast<const void *>(fn), threads, smem), threads, smem, st>>>(
+    fn<<<nsm * resident_ctas(reinterpret_cast<const void *>(fn), threads, smem), threads, smem, st>>>(
         a, g, kc);
     cuda_check(cudaGetLastError(), spread ? "spread launch" : "interpolation launch");
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  }
-  // Resident CTAs an SM, cached: the query is a driver call, and plans enqueue
-  // launches while a stream is being captured into a graph.
-  static int occupancy(const void *fn, int threads, size_t smem) {
-    static std::mutex mu;
-    static std::map<std::tuple<const void *, size_t, int>, int> memo;
-    int dev = 0;
-    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    const auto key = std::make_tuple(fn, smem, dev);
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = memo.find(key);
-    if (it != memo.end()) return it->second;
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, smem);
-    return memo[key] = std::max(nb, 1);
   }
   static void dispatch(int W, bool spread, int nsm, cudaStream_t st, const GridArgs &a,
                        const DevGeom &g, const DevKernel<R> &kc) {
@@ -123,8 +124,10 @@ struct ColKernels {
     constexpr int NB = Cfg::NB;
     EncodeTiledFn enc = encode_tiled();
     if (!err || !enc || env_int("WSG_UCOL_TMA", 1) == 0) return false;
-    if (NB * 2 * int(sizeof(R)) % 16 != 0 || (a.ny / 2) % NB != 0) return false;
-    if (sizeof(R) == 4 && ((a.nv - a.ny / 2) % 2) != 0) return false;
+    if (NB * 2 * int(sizeof(R)) % 16 != 0) return false;
+    // (columns that start inside the row wrap after nv - joff of them)
+    if (a.joff != 0 && (a.nv - a.joff) % NB != 0) return false;
+    if (sizeof(R) == 4 && (a.joff % 2 != 0 || a.nv % 2 != 0)) return false;
     CUtensorMap map;
     const cuuint64_t dims[2] = {cuuint64_t(2) * cuuint64_t(npl) * cuuint64_t(a.nv),
                                 cuuint64_t(a.band_rows)};
@@ -307,6 +310,30 @@ void grid_dispatch(int W, bool spread, int nsm, cudaStream_t st, const GridArgs 
 template <typename R>
 void col_run(int logM, bool bwd, const ColArgs &a, int npl, cudaStream_t st, int *err) {
   ColKernels<R>::run(logM, bwd, a, npl, st, err);
+}
+template <int LOGM>
+void row_run1(bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
+  using Cfg = RowCfg<(1 << LOGM)>;
+  auto *fn = bwd ? k_vrow_bwd<LOGM> : k_vrow_fwd<LOGM>;
+  const size_t smem = Cfg::smem(a.K);
+  require(smem <= kMaxSmemPerBlock, "internal: row transform exceeds shared memory");
+  smem_attr(fn, smem);
+  const int occ = resident_ctas(reinterpret_cast<const void *>(fn), Cfg::THREADS, smem);
+  const long long items = (a.nrow + Cfg::NB - 1) / Cfg::NB;
+  fn<<<unsigned(std::min<long long>(items, (long long)nsm * occ)), Cfg::THREADS, smem, st>>>(a);
+  cuda_check(cudaGetLastError(), "row transform launch");
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
+void row_run(int logM, bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
+  switch (logM) {
+    case 8: row_run1<8>(bwd, a, nsm, st); break;
+    case 9: row_run1<9>(bwd, a, nsm, st); break;
+    case 10: row_run1<10>(bwd, a, nsm, st); break;
+    case 11: row_run1<11>(bwd, a, nsm, st); break;
+    case 12: row_run1<12>(bwd, a, nsm, st); break;
+    case 13: row_run1<13>(bwd, a, nsm, st); break;
+    default: throw std::runtime_error("unsupported pruned FFT length");
+  }
 }
 template <typename R>
 void launch_screen_add(dim3 grid, cudaStream_t st, const ScreenArgs &s, const void *H,

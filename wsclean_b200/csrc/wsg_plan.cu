@@ -56,7 +56,7 @@ Plan::~Plan() {
   for (auto &j : jobs_)
     for (cufftHandle h : {j.fft, j.gfft})
       if (h) cufftDestroy(h);
-  for (DevBuf *b : {&rec_, &chunks_, &chunk_job_, &jobgeom_, &band_, &H_, &img_, &cf_, &tw_,
+  for (DevBuf *b : {&rec_, &chunks_, &chunk_job_, &jobgeom_, &band_, &H_, &hv_, &img_, &cf_, &tw_,
                     &small_, &fftwork_})
     b->release();
 }
@@ -191,7 +191,8 @@ void Plan::build(const std::vector<wsg_job> &js) {
     nchunks_ += nch_j;
     // corrections and twiddles of this grid
     pj.cc = cx_.upload_corrections(gp);
-    const void *twd = gp.ucufft ? nullptr : cx_.upload_twiddles(gp, sizeof(R) == 8);
+    const void *twd = gp.ucufft ? nullptr : cx_.u_tables(gp, sizeof(R) == 8);
+    const void *twv = gp.vprune ? cx_.v_tables(gp) : nullptr;
     CK(cudaStreamSynchronize(st));  // the uploads are stream-ordered
     const size_t ncf = gp.nx / 2 + 1 + gp.ny / 2 + 1;
     pj.cf_off = cf_host.size();
@@ -205,8 +206,14 @@ void Plan::build(const std::vector<wsg_job> &js) {
       tw_host.resize(align256(tw_host.size() + ntw));
       CK(cudaMemcpy(tw_host.data() + pj.tw_off, twd, ntw, cudaMemcpyDeviceToHost));
     }
+    if (gp.vprune) {
+      const size_t ntw = col_table_entries(size_t(1) << gp.logMv, size_t(gp.Kv)) * cs;
+      pj.twv_off = tw_host.size();
+      tw_host.resize(align256(tw_host.size() + ntw));
+      CK(cudaMemcpy(tw_host.data() + pj.twv_off, twv, ntw, cudaMemcpyDeviceToHost));
+    }
     // the job's band grid with all its planes, and its v-FFT plan
-    pj.band_bytes = gp.band_rows * gp.nplanes * gp.nv * cs;
+    pj.band_bytes = gp.band_rows * gp.nplanes * gp.nvs() * cs;
     pj.band_off = band_total_;
     band_total_ = align256(band_total_ + pj.band_bytes);
     max_npix_ = std::max(max_npix_, gp.nx * gp.ny);
@@ -214,14 +221,15 @@ void Plan::build(const std::vector<wsg_job> &js) {
   require(nrec_ > 0, "no active visibilities in any job");
   CK(cudaMemcpyAsync(small_.p, &nchunks_, sizeof(int), cudaMemcpyHostToDevice, st));
 
-  size_t hmax = 0, work = 0;
+  size_t hmax = 0, work = 0, hvmax = 0;
   std::vector<JobGeom> jg(jobs_.size());
   band_.ensure(band_total_);
   for (size_t j = 0; j < jobs_.size(); ++j) {
     PlanJob &pj = jobs_[j];
     if (pj.nrec == 0) continue;
     const GridPlan &gp = pj.gp;
-    if (!gp.ucufft) hmax = std::max(hmax, gp.nplanes * gp.ny * gp.hrow() * cs);
+    if (!gp.ucufft) hmax = std::max(hmax, gp.nplanes * gp.ncol() * gp.hrow() * cs);
+    if (gp.vprune) hvmax = std::max(hvmax, gp.band_rows * gp.nplanes * gp.ncol() * cs);
     JobGeom &g = jg[j];
     g.nu = int(gp.nu);
     g.nv = int(gp.nv);
@@ -231,11 +239,13 @@ void Plan::build(const std::vector<wsg_job> &js) {
     g.P = int(gp.nplanes);
     g.pb0 = 0;
     g.pb1 = int(gp.nplanes);
+    g.Lv = gp.vprune ? int(gp.Lv) : -1;
+    g.nvs = int(gp.nvs());
     g.grid = static_cast<char *>(band_.p) + pj.band_off;
     size_t w = 0;
     if (gp.ucufft) {  // the whole grid: each plane's 2-D transform in place
       pj.gfft = make_grid_fft_plan(gp.nu, gp.nv, gp.nplanes, sizeof(R) == 8, w);
-    } else {
+    } else if (!gp.vprune) {
       CF(cufftCreate(&pj.fft));
       CF(cufftSetAutoAllocation(pj.fft, 0));
       int n = int(gp.nv), inembed = n, onembed = n;
@@ -246,6 +256,7 @@ void Plan::build(const std::vector<wsg_job> &js) {
     work = std::max(work, w);
   }
   H_.ensure(hmax);
+  hv_.ensure(std::max<size_t>(hvmax, 16));
   img_.ensure(max_npix_ * sizeof(double));
   fftwork_.ensure(std::max<size_t>(work, 256));
   jobgeom_.ensure(jg.size() * sizeof(JobGeom));
@@ -298,25 +309,35 @@ void Plan::enqueue_grid(const void *vis, void *const *dirty, int accumulate) {
       exec_grid_fft(pj.gfft, band, gp.nv, gp.nplanes, CUFFT_INVERSE, sizeof(R) == 8, st,
                     fftwork_.p);
     } else {
-      CF(cufftSetStream(pj.fft, st));
-      CF(cufftSetWorkArea(pj.fft, fftwork_.p));
-      if (sizeof(R) == 8)
-        CF(cufftExecZ2Z(pj.fft, reinterpret_cast<cufftDoubleComplex *>(band),
-                        reinterpret_cast<cufftDoubleComplex *>(band), CUFFT_INVERSE));
-      else
-        CF(cufftExecC2C(pj.fft, reinterpret_cast<cufftComplex *>(band),
-                        reinterpret_cast<cufftComplex *>(band), CUFFT_INVERSE));
-      ColArgs ca = make_col(gp, gp.nplanes, static_cast<char *>(tw_.p) + pj.tw_off, band, H_.p);
+      void *cols = band;  // the rows transformed along v
+      if (gp.vprune) {
+        cols = hv_.p;
+        row_run(gp.logMv, true,
+                make_row(gp, gp.nplanes, gp.nplanes, static_cast<char *>(tw_.p) + pj.twv_off, band,
+                         cols),
+                cx_.num_sms, st);
+      } else {
+        CF(cufftSetStream(pj.fft, st));
+        CF(cufftSetWorkArea(pj.fft, fftwork_.p));
+        if (sizeof(R) == 8)
+          CF(cufftExecZ2Z(pj.fft, reinterpret_cast<cufftDoubleComplex *>(band),
+                          reinterpret_cast<cufftDoubleComplex *>(band), CUFFT_INVERSE));
+        else
+          CF(cufftExecC2C(pj.fft, reinterpret_cast<cufftComplex *>(band),
+                          reinterpret_cast<cufftComplex *>(band), CUFFT_INVERSE));
+      }
+      ColArgs ca = make_col(gp, gp.nplanes, static_cast<char *>(tw_.p) + pj.tw_off, cols, H_.p);
       col_run<R>(gp.logM, true, ca, int(gp.nplanes), st, d_err);
     }
+    // the w-screen's sum (all planes at once) goes straight to the caller's
+    // image; accumulating calls go through the FP64 image
+    const int out_mode = accumulate ? 0 : (a_.dirty_type == WSG_F64 ? 2 : 1);
     if (accumulate) {
       if (a_.dirty_type == WSG_F64)
         k_load_image<double><<<nb, 256, 0, st>>>(npix, (const double *)dirty[j], img, 0);
       else
         k_load_image<float><<<nb, 256, 0, st>>>(npix, (const float *)dirty[j], img, 0);
       cuda_check(cudaGetLastError(), "k_load_image launch");
-    } else {
-      CK(cudaMemsetAsync(img, 0, npix * sizeof(double), st));
     }
     ScreenArgs sa = make_screen(gp, reinterpret_cast<const double *>(cf_.p) + pj.cf_off, pj.cc,
                                 gp.nplanes);
@@ -324,15 +345,16 @@ void Plan::enqueue_grid(const void *vis, void *const *dirty, int accumulate) {
     sa.npl = int(gp.nplanes);
     const dim3 sg = screen_grid(gp);
     if (gp.ucufft)
-      launch_screen_add_grid<R>(sg, st, sa, band, img, nullptr, 0);
+      launch_screen_add_grid<R>(sg, st, sa, band, img, dirty[j], out_mode);
     else
-      launch_screen_add<R>(sg, st, sa, H_.p, img, nullptr, 0);
+      launch_screen_add<R>(sg, st, sa, H_.p, img, dirty[j], out_mode);
+    if (!accumulate) continue;
     if (a_.dirty_type == WSG_F64)
       k_store_image<double><<<nb, 256, 0, st>>>(npix, img, (double *)dirty[j]);
     else
       k_store_image<float><<<nb, 256, 0, st>>>(npix, img, (float *)dirty[j]);
     cuda_check(cudaGetLastError(), "k_store_image launch");
-    g_kernel_launches.fetch_add(accumulate ? 3 : 2, std::memory_order_relaxed);
+    g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
   }
   (void)cs;
 }
@@ -351,14 +373,8 @@ void Plan::enqueue_degrid(const void *const *dirty, void *vis) {
     const PlanJob &pj = jobs_[j];
     if (pj.nrec == 0) continue;
     const GridPlan &gp = pj.gp;
-    const size_t npix = gp.nx * gp.ny;
-    double *img = reinterpret_cast<double *>(img_.p);
-    const int nb = launch_blocks(npix, 256);
-    if (a_.dirty_type == WSG_F64)
-      k_load_image<double><<<nb, 256, 0, st>>>(npix, (const double *)dirty[j], img, 0);
-    else
-      k_load_image<float><<<nb, 256, 0, st>>>(npix, (const float *)dirty[j], img, 0);
-    cuda_check(cudaGetLastError(), "k_load_image launch");
+    // the w-screen reads the caller's image in place
+    const int f32 = a_.dirty_type == WSG_F32 ? 1 : 0;
     ScreenArgs sa = make_screen(gp, reinterpret_cast<const double *>(cf_.p) + pj.cf_off, pj.cc,
                                 gp.nplanes);
     sa.pb0 = 0;
@@ -368,24 +384,32 @@ void Plan::enqueue_degrid(const void *const *dirty, void *vis) {
     if (gp.ucufft) {
       // the whole grid, zero outside the image, screened and transformed in place
       CK(cudaMemsetAsync(band, 0, pj.band_bytes, st));
-      launch_screen_put_grid<R>(sg, st, sa, img, 0, band);
+      launch_screen_put_grid<R>(sg, st, sa, dirty[j], f32, band);
       exec_grid_fft(pj.gfft, band, gp.nv, gp.nplanes, CUFFT_FORWARD, sizeof(R) == 8, st,
                     fftwork_.p);
     } else {
-      launch_screen_put<R>(sg, st, sa, img, 0, H_.p);
-      clear_outside_columns(band, gp.band_rows * gp.nplanes, gp.nv, gp.ny, cs, st);
-      ColArgs ca = make_col(gp, gp.nplanes, static_cast<char *>(tw_.p) + pj.tw_off, band, H_.p);
+      launch_screen_put<R>(sg, st, sa, dirty[j], f32, H_.p);
+      void *cols = gp.vprune ? hv_.p : band;
+      if (!gp.vprune)
+        clear_outside_columns(band, gp.band_rows * gp.nplanes, gp.nv, gp.ny, cs, st);
+      ColArgs ca = make_col(gp, gp.nplanes, static_cast<char *>(tw_.p) + pj.tw_off, cols, H_.p);
       col_run<R>(gp.logM, false, ca, int(gp.nplanes), st, d_err);
-      CF(cufftSetStream(pj.fft, st));
-      CF(cufftSetWorkArea(pj.fft, fftwork_.p));
-      if (sizeof(R) == 8)
-        CF(cufftExecZ2Z(pj.fft, reinterpret_cast<cufftDoubleComplex *>(band),
-                        reinterpret_cast<cufftDoubleComplex *>(band), CUFFT_FORWARD));
-      else
-        CF(cufftExecC2C(pj.fft, reinterpret_cast<cufftComplex *>(band),
-                        reinterpret_cast<cufftComplex *>(band), CUFFT_FORWARD));
+      if (gp.vprune) {
+        row_run(gp.logMv, false,
+                make_row(gp, gp.nplanes, gp.nplanes, static_cast<char *>(tw_.p) + pj.twv_off, band,
+                         cols),
+                cx_.num_sms, st);
+      } else {
+        CF(cufftSetStream(pj.fft, st));
+        CF(cufftSetWorkArea(pj.fft, fftwork_.p));
+        if (sizeof(R) == 8)
+          CF(cufftExecZ2Z(pj.fft, reinterpret_cast<cufftDoubleComplex *>(band),
+                          reinterpret_cast<cufftDoubleComplex *>(band), CUFFT_FORWARD));
+        else
+          CF(cufftExecC2C(pj.fft, reinterpret_cast<cufftComplex *>(band),
+                          reinterpret_cast<cufftComplex *>(band), CUFFT_FORWARD));
+      }
     }
-    g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
   }
   CK(cudaMemsetAsync(counter, 0, sizeof(int), st));  // (the error word stays until read)
   GridArgs ga{};
@@ -518,7 +542,7 @@ void Plan::stats(size_t job, wsg_stats &o) const {
   o.dw = g.dw;
   o.nshift = g.nshift;
   o.precision = g.fp32 ? WSG_PREC_MIXED : WSG_PREC_FP64;
-  o.device_bytes = rec_.n + chunks_.n + chunk_job_.n + band_.n + H_.n + img_.n + fftwork_.n;
+  o.device_bytes = rec_.n + chunks_.n + chunk_job_.n + band_.n + H_.n + hv_.n + img_.n + fftwork_.n;
   o.kernel_launches = g_kernel_launches.load();
 }
 

@@ -67,10 +67,12 @@ StreamGridder::StreamGridder(Context &cx, const wsg_args &a, double wmin, double
   choose_grid(g, a.sigma_min, a.sigma_max, default_tile(!dbl_));
   g.fixed = true;
   const size_t cs = dbl_ ? 16 : 8;
-  band_.ensure(g.band_rows * g.nplanes * g.nv * cs);
+  band_.ensure(g.band_rows * g.nplanes * g.nvs() * cs);
+  if (g.vprune) hv_.ensure(g.band_rows * g.nplanes * g.ncol() * cs);
   img_.ensure(g.nx * g.ny * sizeof(double));
   cc_ = cx_.upload_corrections(g);
-  const void *twd = g.ucufft ? nullptr : cx_.upload_twiddles(g, dbl_);
+  const void *twd = g.ucufft ? nullptr : cx_.u_tables(g, dbl_);
+  const void *twv = g.vprune ? cx_.v_tables(g) : nullptr;
   CK(cudaStreamSynchronize(cx_.stream));  // the uploads are stream-ordered
   const size_t ncf = g.nx / 2 + 1 + g.ny / 2 + 1;
   cf_.ensure(ncf * sizeof(double));
@@ -81,13 +83,19 @@ StreamGridder::StreamGridder(Context &cx, const wsg_args &a, double wmin, double
     tw_.ensure(ntw);
     CK(cudaMemcpy(tw_.p, twd, ntw, cudaMemcpyDeviceToDevice));
   }
-  CF(cufftCreate(&fft_));
-  CF(cufftSetAutoAllocation(fft_, 0));
-  int n = int(g.nv), inembed = n, onembed = n;
-  size_t work = 0;
-  CF(cufftMakePlanMany(fft_, 1, &n, &inembed, 1, n, &onembed, 1, n, dbl_ ? CUFFT_Z2Z : CUFFT_C2C,
-                       int(g.band_rows * g.nplanes), &work));
-  fftwork_.ensure(std::max<size_t>(work, 256));
+  if (g.vprune) {
+    const size_t ntw = col_table_entries(size_t(1) << g.logMv, size_t(g.Kv)) * cs;
+    twv_.ensure(ntw);
+    CK(cudaMemcpy(twv_.p, twv, ntw, cudaMemcpyDeviceToDevice));
+  } else {
+    CF(cufftCreate(&fft_));
+    CF(cufftSetAutoAllocation(fft_, 0));
+    int n = int(g.nv), inembed = n, onembed = n;
+    size_t work = 0;
+    CF(cufftMakePlanMany(fft_, 1, &n, &inembed, 1, n, &onembed, 1, n, dbl_ ? CUFFT_Z2Z : CUFFT_C2C,
+                         int(g.band_rows * g.nplanes), &work));
+    fftwork_.ensure(std::max<size_t>(work, 256));
+  }
   if (!g.ucufft) H_.ensure(plane_batch() * row_plane_bytes());
   CK(cudaStreamCreateWithFlags(&copy_, cudaStreamNonBlocking));
   for (auto &sl : slots_) {
@@ -138,14 +146,14 @@ StreamGridder::~StreamGridder() {
     for (DevBuf *d : {&b.uvw, &b.vis, &b.wgt, &b.mask}) d->release();
   }
   if (fft_) cufftDestroy(fft_);
-  for (DevBuf *b : {&band_, &H_, &img_, &cf_, &tw_, &fftwork_, &vout_, &lambda_}) b->release();
+  for (DevBuf *b : {&band_, &H_, &hv_, &img_, &cf_, &tw_, &twv_, &fftwork_, &vout_, &lambda_}) b->release();
 }
 
-// Bytes of one plane's u-transformed rows: ny segmented rows of hrow
+// Bytes of one plane's u-transformed rows: ncol() segmented rows of hrow
 // entries (none with the whole-grid layout, which is screened in place).
 size_t StreamGridder::row_plane_bytes() const {
   const size_t cs = dbl_ ? 16 : 8;
-  return gp_.ucufft ? 0 : gp_.hrow() * gp_.ny * cs;
+  return gp_.ucufft ? 0 : gp_.hrow() * gp_.ncol() * cs;
 }
 
 // Planes per pass of the final transforms (the u-transformed rows of a pass
@@ -363,10 +371,11 @@ void StreamGridder::finish_t(void *dirty, int accumulate) {
     else
       k_load_image<float><<<nb, 256, 0, st>>>(npix, (const float *)din, img, 0);
     cuda_check(cudaGetLastError(), "k_load_image launch");
-  } else {
-    CK(cudaMemsetAsync(img, 0, npix * sizeof(double), st));
   }
-  if (g.ucufft) {
+  if (g.vprune) {
+    row_run(g.logMv, true, make_row(g, g.nplanes, g.nplanes, twv_.p, band_.p, hv_.p), cx_.num_sms,
+            st);
+  } else if (g.ucufft) {
     // the whole grid: each plane's 2-D transform in place, screened in place
     cx_.grid_fft(band_.p, g, g.nplanes, g.nplanes, CUFFT_INVERSE, sizeof(R) == 8);
   } else {
@@ -387,28 +396,35 @@ void StreamGridder::finish_t(void *dirty, int accumulate) {
     CK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
     err_armed_ = true;
   }
+  // one pass and nothing to accumulate: the w-screen's sum goes straight to
+  // the output image, else through the FP64 accumulator
+  void *dout = ddev ? dirty : cx_.b_out.ensure(npix * dsz);
+  const bool direct = !accumulate && P >= g.nplanes;
+  const int out_mode = direct ? (a_.dirty_type == WSG_F64 ? 2 : 1) : 0;
+  if (!accumulate && !direct) CK(cudaMemsetAsync(img, 0, npix * sizeof(double), st));
   for (size_t p0 = 0; p0 < g.nplanes; p0 += P) {
     const size_t np = std::min(P, g.nplanes - p0);
     // the band layout is [row][plane][nv]: a pass starts p0 planes into each row
-    char *band_p0 = static_cast<char *>(band_.p) + p0 * g.nv * cs;
+    char *band_p0 = static_cast<char *>(g.vprune ? hv_.p : band_.p) + p0 * g.nvt() * cs;
     ScreenArgs sa = make_screen(g, reinterpret_cast<const double *>(cf_.p), cc_, g.nplanes);
     sa.pb0 = int(p0);
     sa.npl = int(np);
     const dim3 sg = screen_grid(g);
     if (g.ucufft) {
-      launch_screen_add_grid<R>(sg, st, sa, band_p0, img, nullptr, 0);
+      launch_screen_add_grid<R>(sg, st, sa, band_p0, img, dout, out_mode);
     } else {
       ColArgs ca = make_col(g, g.nplanes, tw_.p, band_p0, H_.p);
       col_run<R>(g.logM, true, ca, int(np), st, d_err);
-      launch_screen_add<R>(sg, st, sa, H_.p, img, nullptr, 0);
+      launch_screen_add<R>(sg, st, sa, H_.p, img, dout, out_mode);
     }
   }
-  void *dout = ddev ? dirty : cx_.b_out.ensure(npix * dsz);
-  if (a_.dirty_type == WSG_F64)
-    k_store_image<double><<<nb, 256, 0, st>>>(npix, img, (double *)dout);
-  else
-    k_store_image<float><<<nb, 256, 0, st>>>(npix, img, (float *)dout);
-  cuda_check(cudaGetLastError(), "k_store_image launch");
+  if (!direct) {
+    if (a_.dirty_type == WSG_F64)
+      k_store_image<double><<<nb, 256, 0, st>>>(npix, img, (double *)dout);
+    else
+      k_store_image<float><<<nb, 256, 0, st>>>(npix, img, (float *)dout);
+    cuda_check(cudaGetLastError(), "k_store_image launch");
+  }
   if (!ddev) CK(cudaMemcpyAsync(dirty, dout, npix * dsz, cudaMemcpyDeviceToHost, st));
   CK(cudaMemsetAsync(band_.p, 0, band_.n, st));
   err_armed_ = false;
@@ -427,20 +443,21 @@ void StreamGridder::finish(void *dirty, int accumulate) {
 }
 
 template <typename R>
-void StreamGridder::predict_begin_t(const double *img) {
+void StreamGridder::predict_begin_t(const void *img, int in_f32) {
   const GridPlan &g = gp_;
   cudaStream_t st = cx_.stream;
   const size_t cs = 2 * sizeof(R);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.ensure(4096)) + 3072);
   CK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-  CK(cudaMemsetAsync(band_.p, 0, band_.n, st));
+  // (the pruned v transform writes every band entry)
+  if (!g.vprune) CK(cudaMemsetAsync(band_.p, 0, band_.n, st));
   if (g.ucufft) {
     // the whole grid (zero outside the image, as cleared above): screened
     // in place, then each plane's 2-D transform in place
     ScreenArgs sa = make_screen(g, reinterpret_cast<const double *>(cf_.p), cc_, g.nplanes);
     sa.pb0 = 0;
     sa.npl = int(g.nplanes);
-    launch_screen_put_grid<R>(screen_grid(g), st, sa, img, 0, band_.p);
+    launch_screen_put_grid<R>(screen_grid(g), st, sa, img, in_f32, band_.p);
     cx_.grid_fft(band_.p, g, g.nplanes, g.nplanes, CUFFT_FORWARD, sizeof(R) == 8);
     cx_.check_device_error(d_err);
     return;
@@ -453,18 +470,24 @@ void StreamGridder::predict_begin_t(const double *img) {
     sa.pb0 = int(p0);
     sa.npl = int(np);
     const dim3 sg = screen_grid(g);
-    launch_screen_put<R>(sg, st, sa, img, 0, H_.p);
-    ColArgs ca = make_col(g, g.nplanes, tw_.p, static_cast<char *>(band_.p) + p0 * g.nv * cs, H_.p);
+    launch_screen_put<R>(sg, st, sa, img, in_f32, H_.p);
+    ColArgs ca = make_col(g, g.nplanes, tw_.p,
+                          static_cast<char *>(g.vprune ? hv_.p : band_.p) + p0 * g.nvt() * cs, H_.p);
     col_run<R>(g.logM, false, ca, int(np), st, d_err);  // (the staged forms report on d_err)
   }
-  CF(cufftSetStream(fft_, st));
-  CF(cufftSetWorkArea(fft_, fftwork_.p));
-  if (sizeof(R) == 8)
-    CF(cufftExecZ2Z(fft_, reinterpret_cast<cufftDoubleComplex *>(band_.p),
-                    reinterpret_cast<cufftDoubleComplex *>(band_.p), CUFFT_FORWARD));
-  else
-    CF(cufftExecC2C(fft_, reinterpret_cast<cufftComplex *>(band_.p),
-                    reinterpret_cast<cufftComplex *>(band_.p), CUFFT_FORWARD));
+  if (g.vprune) {
+    row_run(g.logMv, false, make_row(g, g.nplanes, g.nplanes, twv_.p, band_.p, hv_.p), cx_.num_sms,
+            st);
+  } else {
+    CF(cufftSetStream(fft_, st));
+    CF(cufftSetWorkArea(fft_, fftwork_.p));
+    if (sizeof(R) == 8)
+      CF(cufftExecZ2Z(fft_, reinterpret_cast<cufftDoubleComplex *>(band_.p),
+                      reinterpret_cast<cufftDoubleComplex *>(band_.p), CUFFT_FORWARD));
+    else
+      CF(cufftExecC2C(fft_, reinterpret_cast<cufftComplex *>(band_.p),
+                      reinterpret_cast<cufftComplex *>(band_.p), CUFFT_FORWARD));
+  }
   // a staged copy of the u transform that did not complete (once per model;
   // synchronises the stream)
   cx_.check_device_error(d_err);
@@ -476,17 +499,11 @@ void StreamGridder::predict_begin(const void *dirty) {
   for (auto &b : batch_) b.rows = 0;  // rows added since the last finish are discarded
   const size_t npix = gp_.nx * gp_.ny, dsz = a_.dirty_type == WSG_F64 ? 8 : 4;
   const void *din = cx_.stage_in(dirty, npix * dsz, cx_.b_out);
-  double *img = reinterpret_cast<double *>(img_.p);
-  const int nb = launch_blocks(npix, 256);
-  if (a_.dirty_type == WSG_F64)
-    k_load_image<double><<<nb, 256, 0, cx_.stream>>>(npix, (const double *)din, img, 0);
-  else
-    k_load_image<float><<<nb, 256, 0, cx_.stream>>>(npix, (const float *)din, img, 0);
-  cuda_check(cudaGetLastError(), "k_load_image launch");
+  const int f32 = a_.dirty_type == WSG_F32 ? 1 : 0;  // (read in place by the w-screen)
   if (dbl_)
-    predict_begin_t<double>(img);
+    predict_begin_t<double>(din, f32);
   else
-    predict_begin_t<float>(img);
+    predict_begin_t<float>(din, f32);
   mode_ = 2;
 }
 

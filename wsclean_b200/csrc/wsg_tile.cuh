@@ -60,8 +60,14 @@ __device__ __forceinline__ TileLines tile_lines(const int *bb, int norig, const 
   return t;
 }
 
+// The line's first stored column, from the upper half of where (signed when
+// the band's columns are stored, which number at most 8192).
+__device__ __forceinline__ int line_col(const JobRegs &jr, uint32_t where) {
+  return jr.Lv < 0 ? int(where >> 16) : int(where) >> 16;
+}
+
 // One lane's line: its tile offset, the grid row (null outside the pass or
-// the band) and the first v index.
+// the band) and the first column.
 template <int W, typename C>
 __device__ __forceinline__ C *tile_line(const TileLines &t, const JobRegs &jr, int line, int mp,
                                         int ucorner, int vcorner, int RS, int PS, uint32_t &where) {
@@ -77,11 +83,11 @@ __device__ __forceinline__ C *tile_line(const TileLines &t, const JobRegs &jr, i
     ia = t.lu0 + (line - p * t.nbu);
     ib = t.lv0;
   }
-  where = (uint32_t(jr.wrap_v(vcorner + ib)) << 16) | uint32_t(p * PS + ia * RS + ib);
+  where = (uint32_t(jr.first_col(vcorner + ib)) << 16) | uint32_t(p * PS + ia * RS + ib);
   const int plane = mp + p;
   const int bi = jr.band_row(jr.wrap_u(ucorner + ia));
   if (plane < jr.pb0 || plane >= jr.pb1 || bi < 0) return nullptr;
-  return reinterpret_cast<C *>(jr.grid) + (size_t(bi) * jr.P + (plane - jr.pb0)) * size_t(jr.nv);
+  return reinterpret_cast<C *>(jr.grid) + (size_t(bi) * jr.P + (plane - jr.pb0)) * size_t(jr.nvs);
 }
 
 __device__ __forceinline__ void *shfl_ptr(void *p, int src) {
@@ -138,9 +144,8 @@ __device__ __forceinline__ void tile_flush(C *tile, int RS, int PS, const TileLi
         dst[q] = nullptr;
         if (t.act && i + t.sub < n) {
           x[q] = take_cell(&tile[(wh & 0xffffu) + t.col]);
-          int v = int(wh >> 16) + t.col;
-          v -= v >= jr.nv ? jr.nv : 0;
-          if (rp) dst[q] = rp + v;
+          const int v = jr.next_col(line_col(jr, wh), t.col);
+          if (rp && v >= 0) dst[q] = rp + v;
         }
       }
 #pragma unroll
@@ -182,9 +187,8 @@ __device__ __forceinline__ void tile_stage(C *tile, int RS, int PS, const TileLi
       const C *const rp = reinterpret_cast<const C *>(shfl_ptr(row, src));
       const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
       if (t.act && i + t.sub < n) {
-        int v = int(wh >> 16) + t.col;
-        v -= v >= jr.nv ? jr.nv : 0;
-        copy_cell(&tile[(wh & 0xffffu) + t.col], rp ? rp + v : nullptr, jr.grid);
+        const int v = jr.next_col(line_col(jr, wh), t.col);
+        copy_cell(&tile[(wh & 0xffffu) + t.col], rp && v >= 0 ? rp + v : nullptr, jr.grid);
       }
     }
   }
