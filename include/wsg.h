@@ -71,7 +71,8 @@ int wsg_ctx_destroy(wsg_ctx *ctx);
  * returns to the context's own stream (pass cudaStreamLegacy for the legacy
  * default stream).  Work on the stream before a call is ordered before it. */
 int wsg_ctx_set_stream(wsg_ctx *ctx, void *stream);
-/* Releases the cached device buffers and cuFFT plans (they regrow on demand). */
+/* Releases the cached device buffers and cuFFT plans (they regrow on demand),
+ * the last imaging-weight object's grid among them. */
 int wsg_ctx_release_buffers(wsg_ctx *ctx);
 /* Pipelined mode for wsg_ms2dirty / wsg_dirty2ms (0: off, the default).
  * Every call stages its inputs through one of three buffer slots on a copy

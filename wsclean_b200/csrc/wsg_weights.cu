@@ -18,7 +18,18 @@ ImageWeightsGpu::ImageWeightsGpu(Context &cx, int mode, double robust, size_t wi
   if (H_ % 2) ++H_;
   require(W_ >= 2 && H_ >= 2, "image-weight grid too small");
   CK(cudaSetDevice(cx_.device));
-  grid_.ensure(W_ * (H_ / 2) * sizeof(double));
+  const size_t bytes = W_ * (H_ / 2) * sizeof(double);
+  spare_ = cx_.weight_spare;
+  {
+    // the last object's buffers, unless they are far too large
+    std::lock_guard<std::mutex> lk(spare_->mu);
+    if (spare_->grid.n >= bytes && spare_->grid.n / 4 <= bytes) {
+      std::swap(grid_, spare_->grid);
+      std::swap(sums_, spare_->sums);
+      std::swap(lambda_, spare_->lambda);
+    }
+  }
+  grid_.ensure(bytes);
   sums_.ensure(2 * sizeof(double));
   CK(cudaMemsetAsync(grid_.p, 0, W_ * (H_ / 2) * sizeof(double), cx_.stream));
   CK(cudaMemsetAsync(sums_.p, 0, 2 * sizeof(double), cx_.stream));
@@ -28,6 +39,14 @@ ImageWeightsGpu::ImageWeightsGpu(Context &cx, int mode, double robust, size_t wi
 ImageWeightsGpu::~ImageWeightsGpu() {
   cudaSetDevice(cx_.device);
   cudaStreamSynchronize(cx_.stream);
+  {
+    std::lock_guard<std::mutex> lk(spare_->mu);
+    if (grid_.n > spare_->grid.n) {
+      std::swap(grid_, spare_->grid);
+      std::swap(sums_, spare_->sums);
+      std::swap(lambda_, spare_->lambda);
+    }
+  }
   for (DevBuf *b : {&grid_, &sums_, &lambda_, &in_, &out_}) b->release();
 }
 
