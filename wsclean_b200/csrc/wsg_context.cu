@@ -1,6 +1,8 @@
 // Host orchestration of libwsg: execution contexts, buffer cache, cuFFT plans,
 // and the ms2dirty / dirty2ms drivers (the analogues of ducc0's
 // Params::x2dirty and Params::dirty2x, wgridder.h:1430-1501).
+#include <cub/block/block_radix_sort.cuh>
+#include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_select.cuh>
 #include <thrust/iterator/counting_iterator.h>
@@ -11,6 +13,69 @@ namespace wsg {
 
 // libwsg kernels launched by this process (cuFFT and CUB kernels excluded).
 std::atomic<size_t> g_kernel_launches{0};
+
+// ------------------------------------------------------- small sorts
+//
+// Sort, ranks and chunk starts of a small call in one CTA.  The device-wide
+// sort and selection take nine launches and two clears, each a few
+// microseconds of latency with a handful of blocks at work; up to 16384
+// visibilities fit one CTA's registers.  8.4k visibilities: 47 us of kernels in
+// 9 launches and 2 clears -> 21 us in one; 16k: 36 us.  (Both sorts are stable,
+// so the order is the same.)
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallRadix = 5;  // digit bits (4: the same, 6: 28 us instead of 21)
+constexpr size_t kSmallMax = size_t(kSmallThreads) * 16;
+
+template <int IPT>
+__global__ void __launch_bounds__(kSmallThreads)
+k_small_prep(int n, int nvis, const uint32_t *__restrict__ keys, int end_bit, int bin_shift,
+             int chunk, uint32_t *__restrict__ pos, int *__restrict__ starts,
+             int *__restrict__ nstarts) {
+  using Sort = cub::BlockRadixSort<uint32_t, kSmallThreads, IPT, uint32_t, kSmallRadix>;
+  using Scan = cub::BlockScan<int, kSmallThreads>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ typename Scan::TempStorage scan_tmp;
+  __shared__ uint32_t edge[kSmallThreads];
+  const int t = threadIdx.x;
+  uint32_t key[IPT], idx[IPT];
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int k = t * IPT + i;
+    key[i] = k < n ? keys[k] : 0xffffffffu;  // (sorted behind every key)
+    idx[i] = uint32_t(k);
+  }
+  Sort(*reinterpret_cast<typename Sort::TempStorage *>(smem_raw)).Sort(key, idx, 0, end_bit);
+  edge[t] = key[IPT - 1];
+  __syncthreads();
+  const uint32_t before = t > 0 ? edge[t - 1] : 0u;
+  int flag[IPT], sum = 0;
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int s = t * IPT + i;
+    if (s < n && idx[i] < uint32_t(n)) pos[idx[i]] = uint32_t(s);
+    const uint32_t prev = i > 0 ? key[i - 1] : before;
+    flag[i] = s < nvis && (s == 0 || s % chunk == 0 || (key[i] >> bin_shift) != (prev >> bin_shift));
+    sum += flag[i];
+  }
+  int at, total;
+  Scan(scan_tmp).ExclusiveSum(sum, at, total);
+#pragma unroll
+  for (int i = 0; i < IPT; ++i)
+    if (flag[i]) starts[at++] = t * IPT + i;
+  if (t == 0) *nstarts = total;
+}
+
+template <int IPT>
+static void small_prep(size_t n, size_t nvis, const uint32_t *keys, int end_bit, int bin_shift,
+                       int chunk, uint32_t *pos, int *starts, int *nstarts, cudaStream_t st) {
+  using Sort = cub::BlockRadixSort<uint32_t, kSmallThreads, IPT, uint32_t, kSmallRadix>;
+  constexpr size_t smem = sizeof(typename Sort::TempStorage);
+  smem_attr(k_small_prep<IPT>, smem);
+  k_small_prep<IPT><<<1, kSmallThreads, smem, st>>>(int(n), int(nvis), keys, end_bit, bin_shift,
+                                                    chunk, pos, starts, nstarts);
+  cuda_check(cudaGetLastError(), "k_small_prep launch");
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
 
 // ------------------------------------------------------------ utilities
 
@@ -84,7 +149,7 @@ Context::Context(int dev) {
   CK(cudaStreamCreateWithFlags(&d2h, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&ev_start, &ev_in, &ev_done, &ev_scan, &ev_keys})
     CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-  CK(cudaHostAlloc(&h_scan, sizeof(ScanOut), cudaHostAllocMapped));
+  CK(cudaHostAlloc(&h_scan, sizeof(ScanOut) + 64, cudaHostAllocMapped));  // (and an error word)
   CK(cudaHostGetDevicePointer(&h_scan_dev, h_scan, 0));
   for (auto &sl : slots) CK(cudaEventCreateWithFlags(&sl.free_ev, cudaEventDisableTiming));
   std::memset(&stats, 0, sizeof(stats));
@@ -273,9 +338,19 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
   // reads on the copy stream: its read-back then waits for this call's
   // copies only, not for earlier calls' kernels on the main stream
   cudaStream_t sst = scan_st ? scan_st : stream;
+  ScanOut *d_scan = reinterpret_cast<ScanOut *>(b_small.ensure(4096));
+  // on the main stream, with no error word to keep (a stream's stays from batch
+  // to batch), one upload sets the
+  // initial statistics, clears the counters and the error word and brings f/c
+  // (a few channels); otherwise f/c and the statistics go up apart
+  const bool one =
+      sst == stream && !err_pending && !fovc_buf && !gp.fixed && a.nchan <= kSmallChan;
+  small_zeroed = one;
   DevBuf &fbuf = fovc_buf ? *fovc_buf : b_fovc;
-  double *d_fovc = reinterpret_cast<double *>(fbuf.ensure(a.nchan * sizeof(double)));
-  const size_t small_bytes = sizeof(ScanOut) + a.nchan * sizeof(double);
+  double *d_fovc = reinterpret_cast<double *>(
+      one ? static_cast<char *>(b_small.p) + kOffFovc
+          : static_cast<char *>(fbuf.ensure(a.nchan * sizeof(double))));
+  const size_t small_bytes = std::max<size_t>(4096, sizeof(ScanOut) + a.nchan * sizeof(double));
   if (h_small_cap < small_bytes) {
     if (h_small) CK(cudaFreeHost(h_small));
     h_small = nullptr;
@@ -284,18 +359,25 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
     h_small_cap = small_bytes;
   }
   unsigned char *hsm = reinterpret_cast<unsigned char *>(h_small);
-  std::memcpy(hsm + sizeof(ScanOut), fovc.data(), a.nchan * sizeof(double));
-  CK(cudaMemcpyAsync(d_fovc, hsm + sizeof(ScanOut), a.nchan * sizeof(double),
-                     cudaMemcpyHostToDevice, sst));
+  ScanOut h0{};
+  h0.wmin_bits = 0x7ff0000000000000ull;
+  if (one) {
+    std::memset(hsm, 0, kOffFovc);
+    std::memcpy(hsm, &h0, sizeof h0);
+    std::memcpy(hsm + kOffFovc, fovc.data(), a.nchan * sizeof(double));
+    CK(cudaMemcpyAsync(d_scan, hsm, kOffFovc + a.nchan * sizeof(double), cudaMemcpyHostToDevice,
+                       sst));
+  } else {
+    std::memcpy(hsm + sizeof(ScanOut), fovc.data(), a.nchan * sizeof(double));
+    CK(cudaMemcpyAsync(d_fovc, hsm + sizeof(ScanOut), a.nchan * sizeof(double),
+                       cudaMemcpyHostToDevice, sst));
+    std::memcpy(hsm, &h0, sizeof h0);
+    CK(cudaMemcpyAsync(d_scan, hsm, sizeof(h0), cudaMemcpyHostToDevice, sst));
+  }
   Staged st = s;
   st.fovc = d_fovc;
 
   // scan
-  ScanOut h0{};
-  h0.wmin_bits = 0x7ff0000000000000ull;
-  ScanOut *d_scan = reinterpret_cast<ScanOut *>(b_small.ensure(4096));
-  std::memcpy(hsm, &h0, sizeof h0);
-  CK(cudaMemcpyAsync(d_scan, hsm, sizeof(h0), cudaMemcpyHostToDevice, sst));
   // (off the main stream the caller zeroes the whole output itself)
   void *zero_out = scan_st ? nullptr : vis_out_dev;
   // the sort keys of the expected grid come out of the same pass: the fixed
@@ -403,7 +485,52 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
                    reinterpret_cast<const unsigned char *>(&g) + sizeof g);
   mark("choose_grid");
 
+  // Records per chunk: at most 2048 (a flush of the tile costs as much as
+  // ~100 records, so longer chunks are better where there are enough of
+  // them), and fewer where that would leave SMs idle: four chunks an SM.
+  // k_spread: 32 -> 14 us at 8.4k visibilities (64 a chunk), 91 -> 39 us at
+  // 152k (256 a chunk); from 1.2M on the limit is 2048 as before.
+  const int chunk = gp.batch ? chunk_max
+                             : int(std::min<size_t>(chunk_max, std::max<size_t>(
+                                       chunk_min, gp.nvis / (4 * size_t(num_sms)))));
+  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
+
   // keys (unless the scan wrote them for this grid) + sort
+  if (nvis_tot <= kSmallMax && !gp.wide_keys) {
+    uint32_t *keys = reinterpret_cast<uint32_t *>(ka);
+    if (!keyed) {
+      with_types(a, [&](auto *tw, auto *tv) {
+        using TW = std::remove_pointer_t<decltype(tw)>;
+        using TV = std::remove_pointer_t<decltype(tv)>;
+        launch_keys<TW, TV, uint32_t>(*this, a, st, gridding, g, keys, va);
+      });
+    }
+    int *chunks = reinterpret_cast<int *>(b_chunks.ensure((gp.nvis + 1) * sizeof(int)));
+    auto prep = [&](auto ipt) {
+      small_prep<decltype(ipt)::value>(nvis_tot, gp.nvis, keys, gp.key_bits + 1, 2 * gp.lbits, chunk,
+                                       va, chunks, d_nch, stream);
+    };
+    const size_t per = (nvis_tot + kSmallThreads - 1) / kSmallThreads;
+    if (per <= 3)
+      prep(std::integral_constant<int, 3>{});
+    else if (per <= 6)
+      prep(std::integral_constant<int, 6>{});
+    else if (per <= 9)
+      prep(std::integral_constant<int, 9>{});
+    else if (per <= 12)
+      prep(std::integral_constant<int, 12>{});
+    else
+      prep(std::integral_constant<int, 16>{});
+    void *rec = b_rec.ensure(gp.nvis * sizeof(typename RecOf<R>::type));
+    with_types(a, [&](auto *tw, auto *tv) {
+      using TW = std::remove_pointer_t<decltype(tw)>;
+      using TV = std::remove_pointer_t<decltype(tv)>;
+      launch_ranked_records<R, TW, TV>(gp.nvis, a, st, gridding, g, va, rec, stream);
+    });
+    CK(cudaEventRecord(ev_keys, stream));
+    mark("sort+records-submit");
+    return true;
+  }
   void *kb = b_keys_b.ensure(nvis_tot * 8);
   uint32_t *vb = reinterpret_cast<uint32_t *>(b_vals_b.ensure(nvis_tot * 4));
   const int end_bit = gp.key_bits + 1;
@@ -440,17 +567,8 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
 
   // chunk boundaries
   int *chunks = reinterpret_cast<int *>(b_chunks.ensure((gp.nvis + 1) * sizeof(int)));
-  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
   auto select = [&](auto *kbp) {
     using K = std::remove_pointer_t<decltype(kbp)>;
-    // Records per chunk: at most 2048 (a flush of the tile costs as much as
-    // ~100 records, so longer chunks are better where there are enough of
-    // them), and fewer where that would leave SMs idle: four chunks an SM.
-    // k_spread: 32 -> 14 us at 8.4k visibilities (64 a chunk), 91 -> 39 us at
-    // 152k (256 a chunk); from 1.2M on the limit is 2048 as before.
-    const int chunk = gp.batch ? chunk_max
-                               : int(std::min<size_t>(chunk_max, std::max<size_t>(
-                                         chunk_min, gp.nvis / (4 * size_t(num_sms)))));
     ChunkStartPred<K> pred{kbp, 2 * gp.lbits, chunk};
     thrust::counting_iterator<int> it(0);
     size_t tmp = 0;
@@ -730,7 +848,8 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
-  if (!err_pending) CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));  // sticky while pipelined
+  if (!err_pending && !small_zeroed)
+    CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));  // sticky while pipelined
   GridArgs ga{};
   ga.err = d_err;
   ga.rec = b_rec.p;
@@ -743,6 +862,15 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
 
   const int dir = CUFFT_INVERSE;
   float t_grid = 0, t_fft = 0, t_screen = 0;
+  auto pass_times = [&]() {
+    float t = 0;
+    CK(cudaEventElapsedTime(&t, ev[2], ev[3]));
+    t_grid += t;
+    CK(cudaEventElapsedTime(&t, ev[3], ev[4]));
+    t_fft += t;
+    CK(cudaEventElapsedTime(&t, ev[4], ev[5]));
+    t_screen += t;
+  };
   for (size_t pb0 = 0; pb0 < gp.nplanes; pb0 += P) {
     const size_t npl = std::min(P, gp.nplanes - pb0);
     CK(cudaEventRecord(ev[2], stream));
@@ -752,7 +880,7 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
     } else {
       clear_band(band, rowsP, nv, cs);
     }
-    CK(cudaMemsetAsync(counter, 0, sizeof(int), stream));
+    if (pb0 > 0 || !small_zeroed) CK(cudaMemsetAsync(counter, 0, sizeof(int), stream));
     ga.pb0 = int(pb0);
     ga.pb1 = int(pb0 + npl);
     grid_dispatch<R>(gp.kernel.W, true, num_sms, stream, ga, g, kc);
@@ -784,15 +912,10 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
     else
       launch_screen_add<R>(sg, stream, sa, H, img, direct_out, out_mode);
     CK(cudaEventRecord(ev[5], stream));
-    float t = 0;
-    if (!async_mode) CK(cudaEventSynchronize(ev[5]));
-    if (!async_mode) {
-      CK(cudaEventElapsedTime(&t, ev[2], ev[3]));
-      t_grid += t;
-      CK(cudaEventElapsedTime(&t, ev[3], ev[4]));
-      t_fft += t;
-      CK(cudaEventElapsedTime(&t, ev[4], ev[5]));
-      t_screen += t;
+    // (the last pass is waited for with the error word)
+    if (!async_mode && pb0 + P < gp.nplanes) {
+      CK(cudaEventSynchronize(ev[5]));
+      pass_times();
     }
   }
   float t_prep = 0;
@@ -800,6 +923,7 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
     err_pending = true;
   } else {
     check_device_error(d_err);
+    pass_times();
     CK(cudaEventElapsedTime(&t_prep, ev[0], ev[1]));
   }
   record_stats(gp, true, P);
@@ -865,7 +989,8 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
   int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
   int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
   int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
-  if (!err_pending) CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));  // sticky while pipelined
+  if (!err_pending && !small_zeroed)
+    CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));  // sticky while pipelined
   GridArgs ga{};
   ga.err = d_err;
   ga.rec = b_rec.p;
@@ -884,6 +1009,15 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
 
   const int dir = CUFFT_FORWARD;
   float t_grid = 0, t_fft = 0, t_screen = 0;
+  auto pass_times = [&]() {
+    float t = 0;
+    CK(cudaEventElapsedTime(&t, ev[2], ev[3]));
+    t_screen += t;
+    CK(cudaEventElapsedTime(&t, ev[3], ev[4]));
+    t_fft += t;
+    CK(cudaEventElapsedTime(&t, ev[4], ev[5]));
+    t_grid += t;
+  };
   for (size_t pb0 = 0; pb0 < gp.nplanes; pb0 += P) {
     const size_t npl = std::min(P, gp.nplanes - pb0);
     CK(cudaEventRecord(ev[2], stream));
@@ -925,22 +1059,17 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
       fft_exec(h, bandi, band, dir, dbl);
     }
     CK(cudaEventRecord(ev[4], stream));
-    CK(cudaMemsetAsync(counter, 0, sizeof(int), stream));
+    if (pb0 > 0 || !small_zeroed) CK(cudaMemsetAsync(counter, 0, sizeof(int), stream));
     ga.pb0 = int(pb0);
     ga.pb1 = int(pb0 + npl);
     ga.first_pass = pb0 == 0;
     ga.last_pass = pb0 + npl >= gp.nplanes;
     grid_dispatch<R>(gp.kernel.W, false, num_sms, stream, ga, g, kc);
     CK(cudaEventRecord(ev[5], stream));
-    float t = 0;
-    if (!async_mode) CK(cudaEventSynchronize(ev[5]));
-    if (!async_mode) {
-      CK(cudaEventElapsedTime(&t, ev[2], ev[3]));
-      t_screen += t;
-      CK(cudaEventElapsedTime(&t, ev[3], ev[4]));
-      t_fft += t;
-      CK(cudaEventElapsedTime(&t, ev[4], ev[5]));
-      t_grid += t;
+    // (the last pass is waited for with the error word)
+    if (!async_mode && pb0 + P < gp.nplanes) {
+      CK(cudaEventSynchronize(ev[5]));
+      pass_times();
     }
   }
   if (need_acc) {
@@ -954,6 +1083,7 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
     err_pending = true;
   } else {
     check_device_error(d_err);
+    pass_times();
     CK(cudaEventElapsedTime(&t_prep, ev[0], ev[1]));
   }
   record_stats(gp, false, P);
@@ -967,9 +1097,11 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
 }
 
 void Context::check_device_error(const int *d_err) {
-  int h = 0;
-  CK(cudaMemcpyAsync(&h, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  // (to page-locked memory: a pageable copy holds the host for a staging pass)
+  volatile int *hp = reinterpret_cast<int *>(static_cast<char *>(h_scan) + sizeof(ScanOut));
+  CK(cudaMemcpyAsync(const_cast<int *>(hp), d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
   CK(cudaStreamSynchronize(stream));
+  const int h = *hp;
   if (h & 2) throw std::runtime_error("internal error: a staged copy into shared memory did not complete");
   if (h) throw std::runtime_error("internal error: a visibility record fell outside its tile");
 }

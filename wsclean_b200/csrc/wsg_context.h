@@ -168,6 +168,12 @@ class Context {
   // previous call's scan stream was synchronized
   void *h_small = nullptr;
   size_t h_small_cap = 0;
+  // layout of b_small (bytes): the scan's statistics, then the chunk count,
+  // the chunk counter, the error word, f/c of up to kSmallChan channels
+  static constexpr size_t kOffChunks = 1024, kOffCounter = 2048, kOffErr = 3072, kOffFovc = 3328;
+  static constexpr size_t kSmallChan = (4096 - kOffFovc) / sizeof(double);
+  // prepare() zeroed the counter and the error word with its upload
+  bool small_zeroed = false;
   void finish_call(const wsg_args &a, Slot &sl, cudaStream_t last);
 
   int device = 0;

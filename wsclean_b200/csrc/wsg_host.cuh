@@ -299,6 +299,21 @@ void launch_keys(Context &cx, const wsg_args &a, const Staged &s, bool gridding,
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
+// Records of the nvis active visibilities, built in visibility order and
+// scattered to their sorted positions pos (the inactive visibilities sorted
+// last and are skipped).
+template <typename R, typename TW, typename TV>
+void launch_ranked_records(size_t nvis, const wsg_args &a, const Staged &s, bool gridding,
+                           const DevGeom &g, const uint32_t *pos, void *rec, cudaStream_t st) {
+  const size_t nvis_tot = a.nrows * a.nchan;
+  k_records<R, TV, TW><<<launch_blocks(nvis_tot, 256), 256, 0, st>>>(
+      nvis_tot, nvis, int(a.nchan), pos, s.uvw, s.fovc, reinterpret_cast<const TV *>(s.vis),
+      reinterpret_cast<const TW *>(s.wgt), gridding ? 1 : 0, g,
+      reinterpret_cast<typename RecOf<R>::type *>(rec), s.iw);
+  cuda_check(cudaGetLastError(), "k_records launch");
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
+
 // Records of the nvis active visibilities in sorted order: the sorted
 // positions pos (scratch of nvis_tot entries) from the sort's permutation
 // sidx, then the records built in visibility order and scattered to them
@@ -310,12 +325,8 @@ void launch_records(size_t nvis, const wsg_args &a, const Staged &s, bool griddi
   const size_t nvis_tot = a.nrows * a.nchan;
   k_rank<<<launch_blocks(nvis_tot, 256), 256, 0, st>>>(nvis_tot, sidx, pos);
   cuda_check(cudaGetLastError(), "k_rank launch");
-  k_records<R, TV, TW><<<launch_blocks(nvis_tot, 256), 256, 0, st>>>(
-      nvis_tot, nvis, int(a.nchan), pos, s.uvw, s.fovc, reinterpret_cast<const TV *>(s.vis),
-      reinterpret_cast<const TW *>(s.wgt), gridding ? 1 : 0, g,
-      reinterpret_cast<typename RecOf<R>::type *>(rec), s.iw);
-  cuda_check(cudaGetLastError(), "k_records launch");
-  g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  launch_ranked_records<R, TW, TV>(nvis, a, s, gridding, g, pos, rec, st);
 }
 
 // type-dispatch helpers over (weight type, vis type)
