@@ -858,6 +858,20 @@ __device__ __forceinline__ void col_tail(C *cur, C *oth, const C *tw, int t, C (
 // In-place col_tail: the data in buf, each middle stage reading all its
 // inputs before a barrier and writing back in place; the last stage leaves
 // its outputs in o[q] = X[t + TPF q].
+// Barrier of one FFT's threads (TPF consecutive threads of a CTA of THREADS).
+template <int TPF, int THREADS>
+struct GroupSync {
+  int grp;
+  __device__ __forceinline__ void operator()() const {
+    if constexpr (TPF == THREADS)
+      __syncthreads();
+    else if constexpr (TPF <= 32)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TPF) : "memory");
+  }
+};
+
 struct CtaSync {
   __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
@@ -1503,6 +1517,7 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
   __shared__ __align__(8) uint64_t bar;
   const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
   C *A = bufall + size_t(grp) * BL;
+  const GroupSync<TPF, ColCfg<R, M>::THREADS> sync{grp};
   const int npairs = (a.ny + NB - 1) / NB;
   const int nitems = npairs * npl;
   const C *twB = reinterpret_cast<const C *>(a.twB);
@@ -1573,7 +1588,7 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
           v[q] = cmul(g[q], col_twist<C, TPF>(a, twB, twQ, k2, t, q, M, base));
       }
       C o[16];
-      col_fft_inplace<C, M, TPF, +1>(v, A, tws, t, o);
+      col_fft_inplace<C, M, TPF, +1>(v, A, tws, t, o, sync);
       if (jv) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
@@ -1728,6 +1743,7 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
   __shared__ __align__(8) uint64_t bar;
   const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
   C *A = bufall + size_t(grp) * BL;
+  const GroupSync<TPF, ColCfg<R, M>::THREADS> sync{grp};
   C *band = reinterpret_cast<C *>(a.band);
   const C *twB = reinterpret_cast<const C *>(a.twB);
   const C *twQ = reinterpret_cast<const C *>(a.twQ);
@@ -1785,7 +1801,7 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
         }
       }
       C o[16];
-      col_fft_inplace<C, M, TPF, -1>(v, A, tws, t, o);
+      col_fft_inplace<C, M, TPF, -1>(v, A, tws, t, o, sync);
       if (k2 == 0) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) {

@@ -28,20 +28,6 @@ struct RowArgs {
   const void *twM, *twB, *twQ;   // as ColArgs
 };
 
-// Barrier of one FFT's threads (TPF consecutive threads of a CTA of THREADS).
-template <int TPF, int THREADS>
-struct GroupSync {
-  int grp;
-  __device__ __forceinline__ void operator()() const {
-    if constexpr (TPF == THREADS)
-      __syncthreads();
-    else if constexpr (TPF <= 32)
-      __syncwarp();
-    else
-      asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TPF) : "memory");
-  }
-};
-
 template <int M>
 struct RowCfg {
   using C = ColCfg<float, M>;
