@@ -15,7 +15,7 @@
 // FMA chains, their shared-memory operands and a shuffle reduction for the
 // same work and were bound by latency at one CTA an SM.
 // 2.9M visibilities, W = 14 (1024^2, eps 1e-12): spread 4.59 -> 2.35 ms,
-// interpolation 5.19 -> 2.42 ms (1.07 ms of it the products).
+// interpolation 5.19 -> 2.37 ms (1.07 ms of it the products).
 //
 // A CTA's 16 warps work as two teams of 8 on the two halves of a chunk, on one
 // tile.  A team's warps share every record: the spread splits the output tiles
@@ -219,7 +219,13 @@ k_spread64(GridArgs a, DevGeom g, DevKernel<double> kc) {
   uint32_t *luvs =
       reinterpret_cast<uint32_t *>(spare + NWARP * 32 + 4 * 32 * SST) + team * 64;  // [2][32]
   const RecD *recs = reinterpret_cast<const RecD *>(a.rec);
-  const int colg = tw % NG, rowg = tw / NG;
+  // The warp's place in the team's work.  Place 0 has one column tile more
+  // (W = 14: 25 tiles for 8 warps) and no kernel values to evaluate, only the
+  // records' origins; the teams' places are rotated so that the two warps with
+  // the extra tile are on different schedulers (W = 8, 1.2M visibilities in 5
+  // calls: 248 -> 239 us; W = 14: spread the same, interpolation 2.42 -> 2.37 ms).
+  const int place = K::MG == 1 ? (tw + team) % TW : tw;
+  const int colg = place % NG, rowg = place / NG, share = (place + TW - 1) % TW;
 
   for (int i = tid; i < W * PS; i += NWARP * 32) tile[i] = make_double2(0.0, 0.0);
   spare[tid] = 0.0;
@@ -323,7 +329,7 @@ k_spread64(GridArgs a, DevGeom g, DevKernel<double> kc) {
       if (lane < n) {
         double *row = st + lane * SST;
         const double2 V = spread_value(rr, a);
-        eval64_share<W, TW>(kc, rr, tw, g.do_w, [&](int axis, int piece, double val) {
+        eval64_share<W, TW>(kc, rr, share, g.do_w, [&](int axis, int piece, double val) {
           if (axis == 0) {
             row[SU + piece] = val;
           } else if (axis == 1) {
@@ -334,7 +340,7 @@ k_spread64(GridArgs a, DevGeom g, DevKernel<double> kc) {
           }
         });
       }
-      if (tw == TW - 1) {  // (the warp with the smallest share of values)
+      if (share == TW - 1) {  // (the warp with the smallest share of values)
         uint32_t luv = kSkip;
         if (lane < n) {
           luv = origin64(rr, tu, tv, mp, g.T, a.err);
@@ -386,7 +392,7 @@ k_spread64(GridArgs a, DevGeom g, DevKernel<double> kc) {
     };
 
     const int j0 = s0 + (s1 - s0) * team / 2, j1 = s0 + (s1 - s0) * (team + 1) / 2;
-    auto load = [&](int s) { return load64<W, TW>(recs, s, s < j1, tw, tw == TW - 1); };
+    auto load = [&](int s) { return load64<W, TW>(recs, s, s < j1, share, share == TW - 1); };
     if (j0 < j1) {
       RecD rr = load(j0 + lane);
       stage(rr, min(32, j1 - j0), stg, luvs);
@@ -401,7 +407,7 @@ k_spread64(GridArgs a, DevGeom g, DevKernel<double> kc) {
         consume(min(32, j1 - s), stg + b * 32 * SST, luvs + b * 32);
       }
       commit();
-      if (tw == TW - 1) merge_box(cs, b0, b1, b2, b3, lane);
+      if (share == TW - 1) merge_box(cs, b0, b1, b2, b3, lane);
     }
     __syncthreads();
     const TileLines tln = tile_lines<W>(cs.bb, cs.norig, cs.orig, lane, NWARP);
@@ -449,7 +455,10 @@ k_interp64(GridArgs a, DevGeom g, DevKernel<double> kc) {
   uint32_t *luvs = reinterpret_cast<uint32_t *>(osum + NSUM * 64);
   const RecD *recs = reinterpret_cast<const RecD *>(a.rec);
   const bool direct = a.last_pass && a.first_pass;
-  const int grp = K::SOLO ? 0 : tw;
+  // (places as in the spread: place 0 has one step more and no evaluation)
+  const int place = (tw + team) % TW;
+  const int grp = K::SOLO ? 0 : place;
+  const int share = K::SOLO ? 0 : (place + TW - 1) % TW;
 
   // the lane's cells: rows (p, c) of row tile i, (u, v) of step t
   const int rrow = lane >> 2, kq = lane & 3;
@@ -492,8 +501,8 @@ k_interp64(GridArgs a, DevGeom g, DevKernel<double> kc) {
     auto stage = [&](const RecD &rr, int n, double *st, uint32_t *lv) {
       if (lane < n) {
         double *row = st + lane * IST;
-        if (K::SOLO || tw == TW - 1) lv[lane] = origin64(rr, tu, tv, mp, g.T, a.err);
-        eval64_share<W, NG>(kc, rr, grp, g.do_w, [&](int axis, int piece, double val) {
+        if (K::SOLO || share == TW - 1) lv[lane] = origin64(rr, tu, tv, mp, g.T, a.err);
+        eval64_share<W, NG>(kc, rr, share, g.do_w, [&](int axis, int piece, double val) {
           row[axis == 0 ? IU + piece : (axis == 1 ? IV + piece : piece)] = val;
         });
       }
@@ -604,7 +613,7 @@ k_interp64(GridArgs a, DevGeom g, DevKernel<double> kc) {
       };
       // (three sets of origins: those of the batch before are read by the
       // first two warps while the last warp stages the batch after)
-      auto load = [&](int s) { return load64<W, TW>(recs, s, s < j1, tw, tw == TW - 1); };
+      auto load = [&](int s) { return load64<W, TW>(recs, s, s < j1, share, share == TW - 1); };
       RecD rr = load(j0 + lane);
       stage(rr, min(32, j1 - j0), stg, luvs);
       rr = load(j0 + 32 + lane);
