@@ -855,9 +855,6 @@ __device__ __forceinline__ void col_tail(C *cur, C *oth, const C *tw, int t, C (
   }
 }
 
-// In-place col_tail: the data in buf, each middle stage reading all its
-// inputs before a barrier and writing back in place; the last stage leaves
-// its outputs in o[q] = X[t + TPF q].
 // Barrier of one FFT's threads (TPF consecutive threads of a CTA of THREADS).
 template <int TPF, int THREADS>
 struct GroupSync {
@@ -875,6 +872,10 @@ struct GroupSync {
 struct CtaSync {
   __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
+
+// In-place col_tail: the data in buf, each middle stage reading all its
+// inputs before a barrier and writing back in place; the last stage leaves
+// its outputs in o[q] = X[t + TPF q].
 template <typename C, int M, int NS, int TPF, int SIGN, typename Sync>
 __device__ __forceinline__ void col_tail_inplace(C *buf, const C *tw, int t, C (&o)[16],
                                                  const Sync &sync) {
@@ -951,6 +952,18 @@ __device__ __forceinline__ C col_twist(const ColArgs &a, const C *twB, const C *
   const int b = t + TPF * q;
   const int neg = (!a.band_full && b >= M - a.L) ? 1 : 0;
   return cmul(__ldg(&twQ[(k2 * 16 + q) * 2 + neg]), base);
+}
+
+// The twist factors of passes 1 .. K-1 as one table [k2 - 1][slot] in shared
+// memory (base times factor, multiplied out once a CTA): a twisted point then
+// costs one load and one complex multiplication instead of two of each.
+template <typename C, int M, int THREADS>
+__device__ __forceinline__ void fill_twist(C *dst, const C *twB, const C *twQ, int K, bool band_full) {
+  constexpr int TPF = M / 16;
+  for (int i = threadIdx.x; i < (K - 1) * M; i += THREADS) {
+    const int k2 = 1 + i / M, b = i % M, q = b / TPF, t = b % TPF;
+    dst[i] = cmul(__ldg(&twQ[(k2 * 16 + q) * 2 + (q >= 8 && !band_full)]), __ldg(&twB[k2 * TPF + t]));
+  }
 }
 
 // Copies N table entries to shared memory with all of a thread's loads in
@@ -1063,12 +1076,16 @@ k_ucol_bwd(ColArgs a) {
 // k_ucol_bwd_tma is k_ucol_bwd made persistent: each CTA loops over (plane,
 // column group) items, and while it transforms one, the tensor memory
 // accelerator (cp.async.bulk.tensor, 2-D boxes of NB adjacent columns by up
-// to 256 band rows, no multicast) copies the next item's band columns into a
+// to 128 band rows, no multicast) copies the next item's band columns into a
 // shared staging buffer, completing on an mbarrier.  The band loads then
 // overlap the FFTs instead of stalling each CTA at its start, and the stage
 // twiddles are loaded once per CTA instead of once per column group.  The
 // transforms run in place in one buffer per column (the staging buffer
 // takes the place of the second one).
+// Bound by issue (the FFT's arithmetic and shared-memory accesses), not DRAM:
+// 4096^2, M = 2048, K = 3, 14 planes: 0.99 ms; with barriers of one column's
+// threads instead of the CTA's 0.91, with the twist factors multiplied out
+// (fill_twist) 0.87.
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return uint32_t(__cvta_generic_to_shared(p));
@@ -1117,10 +1134,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 template <typename R, int M>
 struct TmaCfg {
   static constexpr int NB = ColCfg<R, M>::NB;
-  static constexpr int BR = 256;                 // rows per box (M >= 256)
-  static constexpr int ROWS = M + 2 * BR;        // staging rows
+  static constexpr int BR = 128;                 // rows per box
   static constexpr int BOX_BYTES = BR * NB * 2 * int(sizeof(R));
-  static constexpr size_t stage_bytes() { return size_t(ROWS) * NB * 2 * sizeof(R); }
+  // staging rows: whole boxes of the two regions
+  __host__ __device__ static constexpr int rows(int L, bool full) {
+    return full ? M : ((L + 1 + BR - 1) / BR + (L + BR - 1) / BR) * BR;
+  }
+  static constexpr size_t stage_bytes(int L, bool full) {
+    return size_t(rows(L, full)) * NB * 2 * sizeof(R);
+  }
 };
 
 // Boxes of region 1 (rows [0, L] or all rows with the full band).
@@ -1512,7 +1534,7 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
   // the staging buffer starts on a 128-byte boundary (the host adds 128 bytes)
   const uint32_t mis = smem_u32(smem_raw) & 127u;
   C *stage = reinterpret_cast<C *>(smem_raw + (mis ? 128u - mis : 0u));   // [ROWS][NB]
-  C *bufall = stage + size_t(Cfg::ROWS) * NB;                               // [NB][BL]
+  C *bufall = stage + size_t(Cfg::rows(a.L, a.band_full)) * NB;             // [NB][BL]
   C *tws = bufall + size_t(NB) * BL;                                        // [M]
   __shared__ __align__(8) uint64_t bar;
   const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
@@ -1524,13 +1546,8 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
   const C *twQ = reinterpret_cast<const C *>(a.twQ);
   const int reg2 = tma_boxes1(a, M, Cfg::BR) * Cfg::BR;  // first staging row of region 2
   fill_table<C, M, ColCfg<R, M>::THREADS>(tws, reinterpret_cast<const C *>(a.twM));
-  if constexpr (TWS) {  // the twist tables after the stage table (barrier below)
-    C *twBs = tws + M, *twQs = twBs + a.K * TPF;
-    for (int i = threadIdx.x; i < a.K * TPF; i += blockDim.x) twBs[i] = twB[i];
-    for (int i = threadIdx.x; i < a.K * 32; i += blockDim.x) twQs[i] = twQ[i];
-    twB = twBs;
-    twQ = twQs;
-  }
+  C *const twist = tws + M;  // TWS: the twist factors after the stage table (barrier below)
+  if constexpr (TWS) fill_twist<C, M, ColCfg<R, M>::THREADS>(twist, twB, twQ, a.K, a.band_full);
   int item = blockIdx.x;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -1574,13 +1591,8 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
 #pragma unroll
         for (int q = 0; q < 16; ++q) v[q] = g[q];
       } else if constexpr (TWS) {
-        const C base = twB[k2 * TPF + t];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const int b = t + TPF * q;
-          const int neg = (!a.band_full && b >= M - a.L) ? 1 : 0;
-          v[q] = cmul(g[q], cmul(twQ[(k2 * 16 + q) * 2 + neg], base));
-        }
+        for (int q = 0; q < 16; ++q) v[q] = cmul(g[q], twist[(k2 - 1) * M + t + TPF * q]);
       } else {
         const C base = __ldg(&twB[k2 * TPF + t]);
 #pragma unroll
@@ -1704,7 +1716,8 @@ k_ucol_fwd(ColArgs a) {
 // next segment (the next pass, or the first pass of the CTA's next item) is
 // requested as soon as the current one has been read into registers, so it
 // lands while the current pass transforms.  The transforms run in place in
-// one buffer per column.
+// one buffer per column.  Bound as k_ucol_bwd_tma, same sizes: 1.20 ms, column
+// barriers 1.12, twist factors multiplied out 1.08.
 
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes,
                                           uint64_t *bar) {
@@ -1750,13 +1763,8 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
   const int npairs = (a.ny + NB - 1) / NB;
   const int nitems = npairs * npl;
   fill_table<C, M, ColCfg<R, M>::THREADS>(tws, reinterpret_cast<const C *>(a.twM));
-  if constexpr (TWS) {  // the twist tables after the stage table (barrier below)
-    C *twBs = tws + M, *twQs = twBs + a.K * TPF;
-    for (int i = threadIdx.x; i < a.K * TPF; i += blockDim.x) twBs[i] = twB[i];
-    for (int i = threadIdx.x; i < a.K * 32; i += blockDim.x) twQs[i] = twQ[i];
-    twB = twBs;
-    twQ = twQs;
-  }
+  C *const twist = tws + M;  // TWS: the twist factors after the stage table (barrier below)
+  if constexpr (TWS) fill_twist<C, M, ColCfg<R, M>::THREADS>(twist, twB, twQ, a.K, a.band_full);
   int item = blockIdx.x;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -1809,17 +1817,14 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
           acc[q].y += o[q].y;
         }
       } else {
-        const C base = TWS ? twB[k2 * TPF + t] : __ldg(&twB[k2 * TPF + t]);
+        const C base = TWS ? C() : __ldg(&twB[k2 * TPF + t]);
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
           C w;
-          if constexpr (TWS) {
-            const int b = t + TPF * q;
-            const int neg = (!a.band_full && b >= M - a.L) ? 1 : 0;
-            w = cmul(twQ[(k2 * 16 + q) * 2 + neg], base);
-          } else {
+          if constexpr (TWS)
+            w = twist[(k2 - 1) * M + t + TPF * q];
+          else
             w = col_twist<C, TPF>(a, twB, twQ, k2, t, q, M, base);
-          }
           w.y = -w.y;
           const C val = cmul(o[q], w);
           acc[q].x += val.x;

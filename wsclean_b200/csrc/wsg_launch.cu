@@ -139,10 +139,10 @@ struct ColKernels {
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return false;
-    const size_t base = Cfg::stage_bytes() +
+    const size_t base = Cfg::stage_bytes(a.L, a.band_full) +
                         (size_t(NB) * FftBuf<M>::value + M) * 2 * sizeof(R) + 128;
-    // the twist tables go to shared memory too when that costs no resident CTA
-    const size_t extra = size_t(a.K) * (M / 16 + 32) * 2 * sizeof(R);
+    // the twist factors go to shared memory too when that costs no resident CTA
+    const size_t extra = size_t(a.K - 1) * M * 2 * sizeof(R);
     const bool tws = twist_tables_fit(base, extra);
     const size_t smem = tws ? base + extra : base;
     auto *kern = tws ? k_ucol_bwd_tma<R, LOGM, true> : k_ucol_bwd_tma<R, LOGM, false>;
@@ -183,9 +183,9 @@ struct ColKernels {
       return false;
     const size_t base = 128 + (size_t(NB) * a.hseg + size_t(NB) * FftBuf<M>::value + M) * cs;
     if (base > 227 * 1024) return false;
-    // the twist tables go to shared memory too when that costs no resident
+    // the twist factors go to shared memory too when that costs no resident
     // CTA (registers or shared memory, whichever binds)
-    const size_t extra = size_t(a.K) * (M / 16 + 32) * cs;
+    const size_t extra = size_t(a.K - 1) * M * cs;  // (the twist factors multiplied out)
     auto *k0 = k_ucol_fwd_bulk<R, LOGM, false>;
     auto *k1 = k_ucol_fwd_bulk<R, LOGM, true>;
     // resident CTAs of each instantiation at these sizes, memoised (the
@@ -314,11 +314,27 @@ void col_run(int logM, bool bwd, const ColArgs &a, int npl, cudaStream_t st, int
 template <int LOGM>
 void row_run1(bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
   using Cfg = RowCfg<(1 << LOGM)>;
-  auto *fn = bwd ? k_vrow_bwd<LOGM> : k_vrow_fwd<LOGM>;
-  const size_t smem = Cfg::smem(a.K);
-  require(smem <= kMaxSmemPerBlock, "internal: row transform exceeds shared memory");
-  smem_attr(fn, smem);
-  const int occ = resident_ctas(reinterpret_cast<const void *>(fn), Cfg::THREADS, smem);
+  // the twist factors multiplied out when that costs no resident CTA
+  auto pick = [&](bool full, int &occ, size_t &smem) {
+    auto *fn = bwd ? (full ? k_vrow_bwd<LOGM, true> : k_vrow_bwd<LOGM, false>)
+                   : (full ? k_vrow_fwd<LOGM, true> : k_vrow_fwd<LOGM, false>);
+    smem = Cfg::smem(a.K, full);
+    occ = 0;
+    if (smem > kMaxSmemPerBlock) return fn;
+    smem_attr(fn, smem);
+    occ = resident_ctas(reinterpret_cast<const void *>(fn), Cfg::THREADS, smem);
+    return fn;
+  };
+  int occ = 0, occ_full = 0;
+  size_t smem = 0, smem_full = 0;
+  auto *fn = pick(false, occ, smem);
+  auto *fn_full = pick(true, occ_full, smem_full);
+  if (occ_full >= occ) {
+    fn = fn_full;
+    occ = occ_full;
+    smem = smem_full;
+  }
+  require(occ > 0, "internal: row transform exceeds shared memory");
   const long long items = (a.nrow + Cfg::NB - 1) / Cfg::NB;
   fn<<<unsigned(std::min<long long>(items, (long long)nsm * occ)), Cfg::THREADS, smem, st>>>(a);
   cuda_check(cudaGetLastError(), "row transform launch");

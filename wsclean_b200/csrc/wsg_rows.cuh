@@ -10,7 +10,7 @@
 // segments out.  cuFFT transformed whole rows of nv points, three quarters of
 // them zeros, and wrote columns that no image pixel uses.  4096^2 image, 1683
 // rows x 14 planes, 1683 of 6144 columns occupied: 2.3 GB in 0.49 ms, now 1.1 GB
-// in 0.36 ms (forward 0.39); 8192^2, 6.8k rows x 13 planes (14000 points, now
+// in 0.35 ms (forward 0.39); 8192^2, 6.8k rows x 13 planes (14000 points, now
 // 2 x 8192): 8.1 ms, now 6.6 (forward 7.0), and the band grid is cleared in 1.0
 // instead of 2.7 ms.
 #pragma once
@@ -32,26 +32,40 @@ template <int M>
 struct RowCfg {
   using C = ColCfg<float, M>;
   static constexpr int TPF = C::TPF, NB = C::NB, THREADS = C::THREADS;
-  static constexpr size_t smem(int K) {
-    return (size_t(NB) * FftBuf<M>::value + M + size_t(K) * (TPF + 32)) * sizeof(float2);
+  static constexpr size_t smem(int K, bool full) {
+    return (size_t(NB) * FftBuf<M>::value + M + (full ? size_t(K - 1) * M : size_t(K) * (TPF + 32))) *
+           sizeof(float2);
   }
 };
 
-// The CTA's tables in shared memory: stage twiddles [M], twist bases [K][TPF],
-// twist factors [K][16][2].
-template <int M>
+// The CTA's tables in shared memory: stage twiddles [M], then the twist factors
+// [K - 1][M] (FULL) or twist bases [K][TPF] and factors [K][16][2].
+template <int M, bool FULL>
 struct RowTables {
   const float2 *tw, *twB, *twQ;
+  // the twist factor of slot t + TPF q in pass k2 > 0 (base: bases()[k2][t])
+  __device__ __forceinline__ float2 base(int k2, int t) const {
+    return FULL ? float2() : twB[k2 * (M / 16) + t];
+  }
+  __device__ __forceinline__ float2 twist(int k2, int t, int q, float2 base) const {
+    if constexpr (FULL) return twB[(k2 - 1) * M + t + (M / 16) * q];
+    return cmul(twQ[(k2 * 16 + q) * 2 + (q >= 8)], base);
+  }
   __device__ __forceinline__ RowTables(float2 *dst, const RowArgs &a) {
     using Cfg = RowCfg<M>;
     fill_table<float2, M, Cfg::THREADS>(dst, reinterpret_cast<const float2 *>(a.twM));
+    tw = dst;
+    twB = twQ = dst + M;
+    if constexpr (FULL) {
+      fill_twist<float2, M, Cfg::THREADS>(dst + M, reinterpret_cast<const float2 *>(a.twB),
+                                          reinterpret_cast<const float2 *>(a.twQ), a.K, false);
+      return;
+    }
     float2 *b = dst + M, *q = b + a.K * Cfg::TPF;
     for (int i = threadIdx.x; i < a.K * Cfg::TPF; i += Cfg::THREADS)
       b[i] = reinterpret_cast<const float2 *>(a.twB)[i];
     for (int i = threadIdx.x; i < a.K * 32; i += Cfg::THREADS)
       q[i] = reinterpret_cast<const float2 *>(a.twQ)[i];
-    tw = dst;
-    twB = b;
     twQ = q;
   }
 };
@@ -65,7 +79,7 @@ __device__ __forceinline__ int row_col(const RowArgs &a, int b, int q) {
 }
 
 // Band rows -> transformed rows, backward (+).
-template <int LOGM>
+template <int LOGM, bool FULL>
 __global__ void __launch_bounds__(RowCfg<(1 << LOGM)>::THREADS, RowCfg<(1 << LOGM)>::THREADS <= 256 ? 2 : 1)
 k_vrow_bwd(RowArgs a) {
   constexpr int M = 1 << LOGM;
@@ -75,7 +89,7 @@ k_vrow_bwd(RowArgs a) {
   float2 *bufall = reinterpret_cast<float2 *>(smem_raw);
   const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
   float2 *A = bufall + grp * BL;
-  const RowTables<M> tb(bufall + NB * BL, a);
+  const RowTables<M, FULL> tb(bufall + NB * BL, a);
   __syncthreads();
   const GroupSync<TPF, Cfg::THREADS> sync{grp};
   for (long long item = (long long)blockIdx.x * NB; item < a.nrow; item += (long long)gridDim.x * NB) {
@@ -97,10 +111,9 @@ k_vrow_bwd(RowArgs a) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) v[q] = g[q];
       } else {
-        const float2 base = tb.twB[k2 * TPF + t];
+        const float2 base = tb.base(k2, t);
 #pragma unroll
-        for (int q = 0; q < 16; ++q)
-          v[q] = cmul(g[q], cmul(tb.twQ[(k2 * 16 + q) * 2 + (q >= 8)], base));
+        for (int q = 0; q < 16; ++q) v[q] = cmul(g[q], tb.twist(k2, t, q, base));
       }
       float2 o[16];
       col_fft_inplace<float2, M, TPF, +1>(v, A, tb.tw, t, o, sync);
@@ -117,7 +130,7 @@ k_vrow_bwd(RowArgs a) {
 }
 
 // Transformed rows -> band rows, forward (-): the transpose.
-template <int LOGM>
+template <int LOGM, bool FULL>
 __global__ void __launch_bounds__(RowCfg<(1 << LOGM)>::THREADS, RowCfg<(1 << LOGM)>::THREADS <= 256 ? 2 : 1)
 k_vrow_fwd(RowArgs a) {
   constexpr int M = 1 << LOGM;
@@ -127,7 +140,7 @@ k_vrow_fwd(RowArgs a) {
   float2 *bufall = reinterpret_cast<float2 *>(smem_raw);
   const int grp = threadIdx.x / TPF, t = threadIdx.x - grp * TPF;
   float2 *A = bufall + grp * BL;
-  const RowTables<M> tb(bufall + NB * BL, a);
+  const RowTables<M, FULL> tb(bufall + NB * BL, a);
   __syncthreads();
   const GroupSync<TPF, Cfg::THREADS> sync{grp};
   for (long long item = (long long)blockIdx.x * NB; item < a.nrow; item += (long long)gridDim.x * NB) {
@@ -153,10 +166,10 @@ k_vrow_fwd(RowArgs a) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) acc[q] = o[q];
       } else {
-        const float2 base = tb.twB[k2 * TPF + t];
+        const float2 base = tb.base(k2, t);
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
-          float2 w = cmul(tb.twQ[(k2 * 16 + q) * 2 + (q >= 8)], base);
+          float2 w = tb.twist(k2, t, q, base);
           w.y = -w.y;
           const float2 x = cmul(o[q], w);
           acc[q].x += x.x;
