@@ -956,7 +956,8 @@ __device__ __forceinline__ C col_twist(const ColArgs &a, const C *twB, const C *
 
 // The twist factors of passes 1 .. K-1 as one table [k2 - 1][slot] in shared
 // memory (base times factor, multiplied out once a CTA): a twisted point then
-// costs one load and one complex multiplication instead of two of each.
+// costs one load and one complex multiplication instead of two of each, 4 % of
+// a transform.  Taken where its (K - 1) M entries cost no resident CTA.
 template <typename C, int M, int THREADS>
 __device__ __forceinline__ void fill_twist(C *dst, const C *twB, const C *twQ, int K, bool band_full) {
   constexpr int TPF = M / 16;
@@ -1131,9 +1132,9 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 // last box of a region may run past its rows (the copy engine fills rows
 // past the band with zeros) into the region's pad.  With the full band,
 // region 1 holds all M rows.
-template <typename R, int M>
+template <typename R, int M, int COLS = ColCfg<R, M>::NB>
 struct TmaCfg {
-  static constexpr int NB = ColCfg<R, M>::NB;
+  static constexpr int NB = COLS;
   static constexpr int BR = 128;                 // rows per box
   static constexpr int BOX_BYTES = BR * NB * 2 * int(sizeof(R));
   // staging rows: whole boxes of the two regions
@@ -1152,11 +1153,11 @@ __device__ __forceinline__ int tma_boxes1(const ColArgs &a, int M, int BR) {
 
 // Issues the boxes of one item (plane lp, first column j0) into the staging
 // buffer and arms the barrier with their bytes (one thread).
-template <typename R, int M>
+template <typename R, int M, int COLS = ColCfg<R, M>::NB>
 __device__ __forceinline__ void tma_issue_item(const ColArgs &a, const CUtensorMap *map,
                                                typename Cplx<R>::type *stage, uint64_t *bar,
                                                int lp, int j0) {
-  using Cfg = TmaCfg<R, M>;
+  using Cfg = TmaCfg<R, M, COLS>;
   int jx = j0 + a.joff;
   jx -= (jx >= a.nv) ? a.nv : 0;
   const int x = 2 * (lp * a.nv + jx);
@@ -1183,8 +1184,9 @@ __device__ __forceinline__ void col_fft_inplace(C (&v)[16], C *buf, const C *tw,
   col_tail_inplace<C, M, 16, TPF, SIGN>(buf, tw, t, o, sync);
 }
 
-// One-column geometries (M = 4096 and 8192 in FP32, where a CTA of M/16
-// threads takes one image column): k_ucol_bwd_pair gives a CTA two adjacent
+// One-column geometries (in FP32 M = 4096, and 8192 where the kernels of four
+// 2048-point transforms do not apply; a CTA of M/16 threads takes one image
+// column): k_ucol_bwd_pair gives a CTA two adjacent
 // columns, loads both -- 16 bytes a band row instead of 8, half the sectors
 // fetched for the data used -- and transforms them in turn, each in place in
 // its own buffer (the band values of the column in hand stay in registers

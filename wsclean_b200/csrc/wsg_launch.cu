@@ -5,6 +5,7 @@
 #include "wsg_grid32.cuh"
 #include "wsg_grid64.cuh"
 #include "wsg_host.cuh"
+#include "wsg_quad.cuh"
 
 namespace wsg {
 
@@ -117,28 +118,31 @@ struct ColKernels {
   // row of NB columns is a multiple of 16 bytes, column groups start on a
   // 16-byte boundary and do not straddle the wrap of the v axis.  Returns
   // false when not used.
+  static bool column_map(const ColArgs &a, int npl, int NB, int rows, CUtensorMap &map) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc || env_int("WSG_UCOL_TMA", 1) == 0) return false;
+    if (NB * 2 * int(sizeof(R)) % 16 != 0) return false;
+    // (columns that start inside the row wrap after nv - joff of them)
+    if (a.joff != 0 && (a.nv - a.joff) % NB != 0) return false;
+    if (sizeof(R) == 4 && (a.joff % 2 != 0 || a.nv % 2 != 0)) return false;
+    const cuuint64_t dims[2] = {cuuint64_t(2) * cuuint64_t(npl) * cuuint64_t(a.nv),
+                                cuuint64_t(a.band_rows)};
+    const cuuint64_t strides[1] = {cuuint64_t(a.P) * cuuint64_t(a.nv) * 2 * sizeof(R)};
+    const cuuint32_t box[2] = {cuuint32_t(2 * NB), cuuint32_t(rows)};
+    const cuuint32_t estr[2] = {1, 1};
+    return enc(&map,
+               sizeof(R) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+               2, const_cast<void *>(a.band), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  }
   template <int LOGM>
   static bool run_tma(const ColArgs &a, int npl, cudaStream_t st, int *err) {
     constexpr int M = 1 << LOGM;
     using Cfg = TmaCfg<R, M>;
     constexpr int NB = Cfg::NB;
-    EncodeTiledFn enc = encode_tiled();
-    if (!err || !enc || env_int("WSG_UCOL_TMA", 1) == 0) return false;
-    if (NB * 2 * int(sizeof(R)) % 16 != 0) return false;
-    // (columns that start inside the row wrap after nv - joff of them)
-    if (a.joff != 0 && (a.nv - a.joff) % NB != 0) return false;
-    if (sizeof(R) == 4 && (a.joff % 2 != 0 || a.nv % 2 != 0)) return false;
     CUtensorMap map;
-    const cuuint64_t dims[2] = {cuuint64_t(2) * cuuint64_t(npl) * cuuint64_t(a.nv),
-                                cuuint64_t(a.band_rows)};
-    const cuuint64_t strides[1] = {cuuint64_t(a.P) * cuuint64_t(a.nv) * 2 * sizeof(R)};
-    const cuuint32_t box[2] = {cuuint32_t(2 * NB), cuuint32_t(Cfg::BR)};
-    const cuuint32_t estr[2] = {1, 1};
-    if (enc(&map, sizeof(R) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
-            2, const_cast<void *>(a.band), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
+    if (!err || !column_map(a, npl, NB, Cfg::BR, map)) return false;
     const size_t base = Cfg::stage_bytes(a.L, a.band_full) +
                         (size_t(NB) * FftBuf<M>::value + M) * 2 * sizeof(R) + 128;
     // the twist factors go to shared memory too when that costs no resident CTA
@@ -164,6 +168,41 @@ struct ColKernels {
     cuda_check(cudaGetLastError(), "k_ucol_bwd_tma launch");
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return true;
+  }
+  // The mixed 8192-point transforms as four of 2048 points (k_ucol_bwd_quad,
+  // k_ucol_fwd_quad), under the conditions of the staged forms and where the
+  // shared memory suffices: bands up to some 8000 rows, image rows up to some
+  // 3500 K.  Returns false when not used.
+  static bool run_quad(bool bwd, const ColArgs &a, int npl, cudaStream_t st, int *err) {
+    if constexpr (sizeof(R) != 4) {
+      return false;
+    } else {
+      if (!err || env_int("WSG_UCOL_TMA", 1) == 0) return false;
+      int dev = 0, nsm = 148;
+      cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+      cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "attribute");
+      const int grid = int(std::min<long long>((long long)((a.ny + 1) / 2) * npl, nsm));
+      const size_t smem = bwd ? QuadCol::bwd_bytes(a.L, a.band_full, a.K)
+                              : QuadCol::fwd_bytes(a.hseg, a.K);
+      // (16 bytes go to the barrier)
+      if (smem + 16 > kMaxSmemPerBlock) return false;
+      if (bwd) {
+        CUtensorMap map;
+        if (!column_map(a, npl, 2, QuadCol::T::BR, map)) return false;
+        smem_attr(k_ucol_bwd_quad, smem);
+        k_ucol_bwd_quad<<<grid, Quad::THREADS, smem, st>>>(a, map, npl, err);
+      } else {
+        // bulk copies and the 16-byte stores of a pair
+        if (a.hseg % 2 != 0 || a.nv % 2 != 0 || a.joff % 2 != 0 ||
+            ((reinterpret_cast<uintptr_t>(a.H) | reinterpret_cast<uintptr_t>(a.band)) & 15) != 0)
+          return false;
+        smem_attr(k_ucol_fwd_quad, smem);
+        k_ucol_fwd_quad<<<grid, Quad::THREADS, smem, st>>>(a, npl, err);
+      }
+      cuda_check(cudaGetLastError(), bwd ? "k_ucol_bwd_quad launch" : "k_ucol_fwd_quad launch");
+      g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+      return true;
+    }
   }
   // The image-to-band transform with each pass's H-row segments staged by
   // bulk copies (k_ucol_fwd_bulk), when its shared memory fits a CTA.
@@ -251,6 +290,7 @@ struct ColKernels {
   static void run1s(bool bwd, const ColArgs &a, int npl, cudaStream_t st, int *err) {
     constexpr int M = 1 << LOGM;
     using Cfg = ColCfg<R, M>;
+    if (LOGM == 13 && run_quad(bwd, a, npl, st, err)) return;
     if (bwd && run_tma<LOGM>(a, npl, st, err)) return;
     if (!bwd && run_bulk<LOGM>(a, npl, st, err)) return;
     if constexpr (sizeof(R) == 4 && Cfg::NB == 1) {
@@ -340,6 +380,17 @@ void row_run1(bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
   cuda_check(cudaGetLastError(), "row transform launch");
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
+// 8192 points: four of 2048 (k_vrow_fwd_quad stages a whole transformed row,
+// and rows of more than some 16000 entries stay with k_vrow_fwd).
+void row_run_quad(bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
+  const size_t smem = bwd ? QuadRow::bwd_bytes(a.K) : QuadRow::fwd_bytes(a.ncol, a.K);
+  if (smem > kMaxSmemPerBlock) return row_run1<13>(bwd, a, nsm, st);
+  auto *fn = bwd ? k_vrow_bwd_quad : k_vrow_fwd_quad;
+  smem_attr(fn, smem);
+  fn<<<unsigned(std::min<long long>(a.nrow, nsm)), Quad::THREADS, smem, st>>>(a);
+  cuda_check(cudaGetLastError(), "row transform launch");
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
 void row_run(int logM, bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
   switch (logM) {
     case 8: row_run1<8>(bwd, a, nsm, st); break;
@@ -347,7 +398,7 @@ void row_run(int logM, bool bwd, const RowArgs &a, int nsm, cudaStream_t st) {
     case 10: row_run1<10>(bwd, a, nsm, st); break;
     case 11: row_run1<11>(bwd, a, nsm, st); break;
     case 12: row_run1<12>(bwd, a, nsm, st); break;
-    case 13: row_run1<13>(bwd, a, nsm, st); break;
+    case 13: row_run_quad(bwd, a, nsm, st); break;
     default: throw std::runtime_error("unsupported pruned FFT length");
   }
 }

@@ -11,8 +11,8 @@
 // them zeros, and wrote columns that no image pixel uses.  4096^2 image, 1683
 // rows x 14 planes, 1683 of 6144 columns occupied: 2.3 GB in 0.49 ms, now 1.1 GB
 // in 0.35 ms (forward 0.39); 8192^2, 6.8k rows x 13 planes (14000 points, now
-// 2 x 8192): 8.1 ms, now 6.6 (forward 7.0), and the band grid is cleared in 1.0
-// instead of 2.7 ms.
+// 2 x 8192, k_vrow_bwd_quad): 8.1 ms, now 5.9 (forward 6.5), and the band grid
+// is cleared in 1.0 instead of 2.7 ms.
 #pragma once
 
 #include "wsg_device.cuh"
