@@ -155,6 +155,7 @@ inline ScreenArgs make_screen(const GridPlan &g, const double *d_cf, const ChebC
   s.ncol = int(g.ncol());
   s.Kv = g.vprune ? g.Kv : 1;
   s.hsegv = int(g.hsegv());
+  s.hsegv_inv = 1.0f / float(s.hsegv);
   s.hm0v = g.vprune ? g.hm0v() : -int(g.ny / 2);
   s.nu = int(g.nu);
   s.nv = int(g.nv);
@@ -176,7 +177,7 @@ inline ScreenArgs make_screen(const GridPlan &g, const double *d_cf, const ChebC
   s.cfu = d_cf;
   s.cfv = d_cf + g.nx / 2 + 1;
   s.ncheb = cc.n;
-  s.ymax = cc.ymax;
+  s.yscale = 2.0 / cc.ymax;
   for (int i = 0; i < cc.n && i < kDMaxCheb; ++i) s.cheb[i] = cc.c[i];
   return s;
 }
