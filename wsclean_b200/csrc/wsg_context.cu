@@ -488,7 +488,7 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
   // Records per chunk: at most 2048 (a flush of the tile costs as much as
   // ~100 records, so longer chunks are better where there are enough of
   // them), and fewer where that would leave SMs idle: four chunks an SM.
-  // k_spread: 32 -> 14 us at 8.4k visibilities (64 a chunk), 91 -> 39 us at
+  // The spread: 32 -> 14 us at 8.4k visibilities (64 a chunk), 91 -> 39 us at
   // 152k (256 a chunk); from 1.2M on the limit is 2048 as before.
   const int chunk = gp.batch ? chunk_max
                              : int(std::min<size_t>(chunk_max, std::max<size_t>(

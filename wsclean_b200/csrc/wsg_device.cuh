@@ -15,7 +15,9 @@
 //               footprint origin repeats, commit to a shared-memory tile, and
 //               flush the tile to the u-band grid with vector atomics
 //                                                             (x2grid_c_helper/HelperX2g2, wgridder.h:934-1031,1142-1236)
-//   cuFFT       backward FFT along v of the occupied u band (all planes of a pass)
+//   k_vrow_bwd  pruned backward FFT along v of the occupied u band, all planes of a
+//               pass (wsg_rows.cuh; cuFFT over whole rows in FP64 and where nv
+//               is not K 2^m)
 //   k_ucol_bwd  pruned backward FFT along u of the image columns only: nu = K M,
 //               K twisted M-point FFTs per column, band in, image rows out
 //                                                             (grid2dirty_c_overwrite_wscreen_add, :496-534)
