@@ -398,7 +398,7 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
     using TW = std::remove_pointer_t<decltype(tw)>;
     using TV = std::remove_pointer_t<decltype(tv)>;
     if (have_spec) {
-      const int nb = std::min(launch_blocks(a.nrows, 256), num_sms * 8);
+      const int nb = std::min(launch_blocks(nvis_tot, 256), num_sms * 8);
       auto go = [&](auto *kp) {
         using K = std::remove_pointer_t<decltype(kp)>;
         k_scan_keys<TV, TW, K><<<nb, 256, 0, sst>>>(

@@ -221,6 +221,35 @@ __device__ __forceinline__ double weighted(const ImgW &iw, const double *__restr
 
 // --------------------------------------------------------------- k_scan
 
+// A thread's visibilities, in visibility order over the grid: lanes take
+// consecutive channels, so that loads of visibilities and weights and stores of
+// keys are coalesced; row and channel are stepped without a division.
+// (Bound by the latency of its loads; a thread used to walk a row's channels,
+// every lane in another row.  8.1M visibilities: 106 -> 78 us, degridding 85 ->
+// 71; 2.9M complex128: 48 -> 30.)
+struct VisWalk {
+  size_t r, dr;
+  int c, dc, nchan;
+  __device__ __forceinline__ explicit VisWalk(int nchan_)
+      : r(~size_t(0)), dr(0), c(0), dc(0), nchan(nchan_) {
+    if (nchan <= 0) return;  // (no visibilities)
+    const size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    const size_t n = size_t(gridDim.x) * blockDim.x;
+    r = k / uint32_t(nchan);
+    c = int(k - r * uint32_t(nchan));
+    dr = n / uint32_t(nchan);
+    dc = int(n - dr * uint32_t(nchan));
+  }
+  __device__ __forceinline__ void next() {
+    r += dr;
+    c += dc;
+    if (c >= nchan) {
+      c -= nchan;
+      ++r;
+    }
+  }
+};
+
 // Active mask, |w| range, max |u|, |v| and the active count of the
 // visibilities (scanData, wgridder.h:1578-1618); with KEYS, also the sort
 // key of every visibility for the grid geometry g, as k_keys writes it (the
@@ -235,44 +264,42 @@ __device__ __forceinline__ void scan_rows(size_t nrows, int nchan, const double 
                                           uint32_t *__restrict__ vals, const ImgW &iw) {
   double lwmin = 1e300, lwmax = 0, lumax = 0, lvmax = 0;
   unsigned long long cnt = 0;
-  for (size_t r = blockIdx.x * size_t(blockDim.x) + threadIdx.x; r < nrows;
-       r += size_t(gridDim.x) * blockDim.x) {
-    double u = uvw[3 * r], v = vfac * uvw[3 * r + 1], w = uvw[3 * r + 2];
-    for (int c = 0; c < nchan; ++c) {
-      size_t k = r * nchan + c;
-      bool act;
-      if (gridding) {
-        TV x = vis[k];
-        auto n = x.x * x.x + x.y * x.y;
-        if (iw.grid)
-          n *= decltype(n)(weighted<TW>(iw, uvw, r, c, wgt ? double(wgt[k]) : 1.0));
-        else if (wgt)
-          n *= wgt[k];
-        if (mask) n *= mask[k];
-        act = (n != 0);
-      } else {
-        act = (!wgt || wgt[k] != 0) && (!mask || mask[k] != 0);
-        if (!act && vis_out) vis_out[k] = TV{0, 0};
-      }
-      K key = KEYS ? K(g.inactive_key) : K(0);
-      if (act) {
-        double f = fovc[c];
-        double aw = fabs(w * f);
-        lwmin = fmin(lwmin, aw);
-        lwmax = fmax(lwmax, aw);
-        lumax = fmax(lumax, fabs(u * f));
-        lvmax = fmax(lvmax, fabs(v * f));
-        ++cnt;
-        if constexpr (KEYS) {
-          VisPix p;
-          vis_pixel(g, u * f, v * f, w * f, p);
-          key = bin_key<K>(g, p);
-        }
-      }
+  for (VisWalk a(nchan); a.r < nrows; a.next()) {
+    const size_t r = a.r, k = r * nchan + a.c;
+    const int c = a.c;
+    const double u = uvw[3 * r], v = vfac * uvw[3 * r + 1], w = uvw[3 * r + 2];
+    bool act;
+    if (gridding) {
+      TV x = vis[k];
+      auto n = x.x * x.x + x.y * x.y;
+      if (iw.grid)
+        n *= decltype(n)(weighted<TW>(iw, uvw, r, c, wgt ? double(wgt[k]) : 1.0));
+      else if (wgt)
+        n *= wgt[k];
+      if (mask) n *= mask[k];
+      act = (n != 0);
+    } else {
+      act = (!wgt || wgt[k] != 0) && (!mask || mask[k] != 0);
+      if (!act && vis_out) vis_out[k] = TV{0, 0};
+    }
+    K key = KEYS ? K(g.inactive_key) : K(0);
+    if (act) {
+      double f = fovc[c];
+      double aw = fabs(w * f);
+      lwmin = fmin(lwmin, aw);
+      lwmax = fmax(lwmax, aw);
+      lumax = fmax(lumax, fabs(u * f));
+      lvmax = fmax(lvmax, fabs(v * f));
+      ++cnt;
       if constexpr (KEYS) {
-        keys[k] = key;
-        vals[k] = uint32_t(k);
+        VisPix p;
+        vis_pixel(g, u * f, v * f, w * f, p);
+        key = bin_key<K>(g, p);
       }
+    }
+    if constexpr (KEYS) {
+      keys[k] = key;
+      vals[k] = uint32_t(k);
     }
   }
   // warp then block reduction
@@ -283,7 +310,26 @@ __device__ __forceinline__ void scan_rows(size_t nrows, int nchan, const double 
     lvmax = fmax(lvmax, __shfl_xor_sync(0xffffffffu, lvmax, o));
     cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
   }
-  if ((threadIdx.x & 31) == 0 && cnt > 0) {
+  __shared__ double red[4][32];
+  __shared__ unsigned long long redn[32];
+  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    red[0][wid] = lwmin;
+    red[1][wid] = lwmax;
+    red[2][wid] = lumax;
+    red[3][wid] = lvmax;
+    redn[wid] = cnt;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int i = 1; i < nw; ++i) {
+    lwmin = fmin(lwmin, red[0][i]);
+    lwmax = fmax(lwmax, red[1][i]);
+    lumax = fmax(lumax, red[2][i]);
+    lvmax = fmax(lvmax, red[3][i]);
+    cnt += redn[i];
+  }
+  if (cnt > 0) {
     atomicMin(&out->wmin_bits, (unsigned long long)__double_as_longlong(lwmin));
     atomicMax(&out->wmax_bits, (unsigned long long)__double_as_longlong(lwmax));
     atomicMax(&out->umax_bits, (unsigned long long)__double_as_longlong(lumax));
@@ -325,34 +371,32 @@ __global__ void k_keys(size_t nrows, int nchan, const double *__restrict__ uvw,
                        const TW *__restrict__ wgt, const uint8_t *__restrict__ mask,
                        int gridding, DevGeom g, K *__restrict__ keys,
                        uint32_t *__restrict__ vals, ImgW iw) {
-  for (size_t r = blockIdx.x * size_t(blockDim.x) + threadIdx.x; r < nrows;
-       r += size_t(gridDim.x) * blockDim.x) {
-    double u = uvw[3 * r], v = g.vfac * uvw[3 * r + 1], w = uvw[3 * r + 2];
-    for (int c = 0; c < nchan; ++c) {
-      size_t k = r * nchan + c;
-      bool act;
-      if (gridding) {
-        TV x = vis[k];
-        auto n = x.x * x.x + x.y * x.y;
-        if (iw.grid)
-          n *= decltype(n)(weighted<TW>(iw, uvw, r, c, wgt ? double(wgt[k]) : 1.0));
-        else if (wgt)
-          n *= wgt[k];
-        if (mask) n *= mask[k];
-        act = (n != 0);
-      } else {
-        act = (!wgt || wgt[k] != 0) && (!mask || mask[k] != 0);
-      }
-      K key = K(g.inactive_key);
-      if (act) {
-        double f = fovc[c];
-        VisPix p;
-        vis_pixel(g, u * f, v * f, w * f, p);
-        key = bin_key<K>(g, p);
-      }
-      keys[k] = key;
-      vals[k] = uint32_t(k);
+  for (VisWalk a(nchan); a.r < nrows; a.next()) {
+    const size_t r = a.r, k = r * nchan + a.c;
+    const int c = a.c;
+    const double u = uvw[3 * r], v = g.vfac * uvw[3 * r + 1], w = uvw[3 * r + 2];
+    bool act;
+    if (gridding) {
+      TV x = vis[k];
+      auto n = x.x * x.x + x.y * x.y;
+      if (iw.grid)
+        n *= decltype(n)(weighted<TW>(iw, uvw, r, c, wgt ? double(wgt[k]) : 1.0));
+      else if (wgt)
+        n *= wgt[k];
+      if (mask) n *= mask[k];
+      act = (n != 0);
+    } else {
+      act = (!wgt || wgt[k] != 0) && (!mask || mask[k] != 0);
     }
+    K key = K(g.inactive_key);
+    if (act) {
+      double f = fovc[c];
+      VisPix p;
+      vis_pixel(g, u * f, v * f, w * f, p);
+      key = bin_key<K>(g, p);
+    }
+    keys[k] = key;
+    vals[k] = uint32_t(k);
   }
 }
 

@@ -278,7 +278,7 @@ void launch_screen_put_grid(dim3 grid, cudaStream_t st, const ScreenArgs &s, con
 template <typename TW, typename TV>
 void launch_scan(Context &cx, const wsg_args &a, const Staged &s, bool gridding, TV *vis_out,
                  ScanOut *d_out, cudaStream_t st) {
-  int nb = launch_blocks(a.nrows, 256);
+  int nb = launch_blocks(a.nrows * a.nchan, 256);
   nb = std::min(nb, cx.num_sms * 8);
   k_scan<TV, TW><<<nb, 256, 0, st>>>(
       a.nrows, int(a.nchan), s.uvw, s.fovc, reinterpret_cast<const TV *>(s.vis),
@@ -291,7 +291,7 @@ void launch_scan(Context &cx, const wsg_args &a, const Staged &s, bool gridding,
 template <typename TW, typename TV, typename K>
 void launch_keys(Context &cx, const wsg_args &a, const Staged &s, bool gridding, const DevGeom &g,
                  K *keys, uint32_t *vals) {
-  int nb = launch_blocks(a.nrows, 256);
+  int nb = launch_blocks(a.nrows * a.nchan, 256);
   k_keys<TV, TW, K><<<nb, 256, 0, cx.stream>>>(a.nrows, int(a.nchan), s.uvw, s.fovc,
                                                reinterpret_cast<const TV *>(s.vis),
                                                reinterpret_cast<const TW *>(s.wgt), s.mask,

@@ -196,7 +196,7 @@ void ms2dirty_noalloc(const wsg_args &a, const void *vis, void *dirty, cudaStrea
   cuda_check(cudaMemcpyAsync(d_scan, &h0, sizeof(h0), cudaMemcpyHostToDevice, stream), "scan init");
   cuda_check(cudaMemsetAsync(d_nch, 0, 3 * sizeof(int), stream), "counters");
   {
-    int nb = std::min(launch_blocks(a.nrows, 256), nsm * 8);
+    int nb = std::min(launch_blocks(nvis_tot, 256), nsm * 8);
     with_types(a, [&](auto *tw, auto *tv) {
       using TW = std::remove_pointer_t<decltype(tw)>;
       using TV = std::remove_pointer_t<decltype(tv)>;
@@ -252,7 +252,7 @@ void ms2dirty_noalloc(const wsg_args &a, const void *vis, void *dirty, cudaStrea
     with_types(a, [&](auto *tw, auto *tv) {
       using TW = std::remove_pointer_t<decltype(tw)>;
       using TV = std::remove_pointer_t<decltype(tv)>;
-      k_keys<TV, TW, uint32_t><<<launch_blocks(a.nrows, 256), 256, 0, stream>>>(
+      k_keys<TV, TW, uint32_t><<<launch_blocks(nvis_tot, 256), 256, 0, stream>>>(
           a.nrows, int(a.nchan), st.uvw, st.fovc, reinterpret_cast<const TV *>(st.vis),
           reinterpret_cast<const TW *>(st.wgt), st.mask, 1, g, ka, va, ImgW{});
     });
