@@ -56,7 +56,7 @@ struct DevGeom {
   int wide;                               // 64-bit sort keys
   unsigned long long inactive_key;
   int Lu, band_rows, band_full;
-  int Lv, nvs;   // occupied v columns stored [-Lv, Lv], nvs a row (Lv < 0: all nv)
+  int Lv, nvs;   // v columns stored: [-Lv, Lv], nvs a row (all nv: Lv = 0)
 };
 
 struct ScanOut {
@@ -592,19 +592,11 @@ struct JobRegs {
     v += (v < 0) ? nv : 0;
     return v - ((v >= nv) ? nv : 0);
   }
-  // Stored column of v where a tile line starts (the columns after it are
-  // checked by next_col; far outside the band, a column that stays outside
-  // over a line's 32 cells), and of a cell c further on, or -1 outside.
-  __device__ __forceinline__ int first_col(int v) const {
-    v = wrap_v(v);
-    if (Lv < 0) return v;
-    v = (v > nv / 2 ? v - nv : v) + Lv;
-    return min(max(v, -64), nvs);
-  }
+  // Stored column of v where a tile line starts, and of a cell c further on
+  // (-1 outside the row).
+  __device__ __forceinline__ int first_col(int v) const { return band_col(wrap_v(v), Lv, nv); }
   __device__ __forceinline__ int next_col(int first, int c) const {
-    const int v = first + c;
-    if (Lv < 0) return v - (v >= nv ? nv : 0);
-    return unsigned(v) < unsigned(nvs) ? v : -1;
+    return band_col_next(first, c, nv, nvs);
   }
 };
 

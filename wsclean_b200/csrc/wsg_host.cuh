@@ -84,7 +84,7 @@ inline DevGeom make_geom(const GridPlan &g) {
   d.Lu = int(g.Lu);
   d.band_rows = int(g.band_rows);
   d.band_full = g.band_full;
-  d.Lv = g.vprune ? int(g.Lv) : -1;
+  d.Lv = g.vprune ? int(g.Lv) : 0;
   d.nvs = int(g.nvs());
   return d;
 }

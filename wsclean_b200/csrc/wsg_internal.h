@@ -34,6 +34,19 @@ inline void require(bool ok, const std::string &msg) {
   if (!ok) throw InvalidArgument(msg);
 }
 
+// Stored columns of a band grid row.  The band grid keeps the v columns
+// -Lv .. Lv of nv, v at (v + Lv) mod nv, nvs entries a row (all columns: Lv = 0,
+// nvs = nv).  A tile line starts at the column band_col gives for a wrapped v
+// and steps on from there modulo nv: next to v = nv / 2 a tile can hold
+// footprints of both ends of the band, whose columns are the row's last and
+// first ones.
+constexpr int band_col(int v, int Lv, int nv) { return v + Lv - (v + Lv >= nv ? nv : 0); }
+// ... of the cell c (< nv) further on, or -1 outside the row.
+constexpr int band_col_next(int first, int c, int nv, int nvs) {
+  const int v = first + c - (first + c >= nv ? nv : 0);
+  return v < nvs ? v : -1;
+}
+
 // One row of the generated ES kernel table.
 struct KernelSpec {
   int W;

@@ -239,7 +239,7 @@ void Plan::build(const std::vector<wsg_job> &js) {
     g.P = int(gp.nplanes);
     g.pb0 = 0;
     g.pb1 = int(gp.nplanes);
-    g.Lv = gp.vprune ? int(gp.Lv) : -1;
+    g.Lv = gp.vprune ? int(gp.Lv) : 0;
     g.nvs = int(gp.nvs());
     g.grid = static_cast<char *>(band_.p) + pj.band_off;
     size_t w = 0;

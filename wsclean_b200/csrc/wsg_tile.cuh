@@ -60,14 +60,9 @@ __device__ __forceinline__ TileLines tile_lines(const int *bb, int norig, const 
   return t;
 }
 
-// The line's first stored column, from the upper half of where (signed when
-// the band's columns are stored, which number at most 8192).
-__device__ __forceinline__ int line_col(const JobRegs &jr, uint32_t where) {
-  return jr.Lv < 0 ? int(where >> 16) : int(where) >> 16;
-}
-
-// One lane's line: its tile offset, the grid row (null outside the pass or
-// the band) and the first column.
+// One lane's line: the grid row (null outside the pass or the band), and in
+// where the first stored column (upper half; grids are below 65535) and the
+// line's tile offset.
 template <int W, typename C>
 __device__ __forceinline__ C *tile_line(const TileLines &t, const JobRegs &jr, int line, int mp,
                                         int ucorner, int vcorner, int RS, int PS, uint32_t &where) {
@@ -144,7 +139,7 @@ __device__ __forceinline__ void tile_flush(C *tile, int RS, int PS, const TileLi
         dst[q] = nullptr;
         if (t.act && i + t.sub < n) {
           x[q] = take_cell(&tile[(wh & 0xffffu) + t.col]);
-          const int v = jr.next_col(line_col(jr, wh), t.col);
+          const int v = jr.next_col(int(wh >> 16), t.col);
           if (rp && v >= 0) dst[q] = rp + v;
         }
       }
@@ -187,7 +182,7 @@ __device__ __forceinline__ void tile_stage(C *tile, int RS, int PS, const TileLi
       const C *const rp = reinterpret_cast<const C *>(shfl_ptr(row, src));
       const uint32_t wh = __shfl_sync(0xffffffffu, where, src);
       if (t.act && i + t.sub < n) {
-        const int v = jr.next_col(line_col(jr, wh), t.col);
+        const int v = jr.next_col(int(wh >> 16), t.col);
         copy_cell(&tile[(wh & 0xffffu) + t.col], rp && v >= 0 ? rp + v : nullptr, jr.grid);
       }
     }
