@@ -1600,11 +1600,7 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
   __syncthreads();  // the barrier is initialised before anyone waits on it
   for (uint32_t parity = 0; item < nitems; item += gridDim.x, parity ^= 1u) {
     const int lp = item / npairs, j = (item % npairs) * NB + grp;
-    if (!mbar_wait(&bar, parity)) {  // the copy did not complete: report and stop
-      if (threadIdx.x == 0) atomicOr(err, 2);
-      mbar_wait(&bar, parity);
-      return;
-    }
+    const bool ok = mbar_wait(&bar, parity);
     // the untwisted band values at slots t + TPF q (zero between the halves)
     C g[16];
 #pragma unroll
@@ -1617,7 +1613,14 @@ k_ucol_bwd_tma(ColArgs a, const __grid_constant__ CUtensorMap tmap, int npl, int
       else if (b >= M - a.L)
         g[q] = stage[size_t(reg2 + b - (M - a.L)) * NB + grp];
     }
-    __syncthreads();  // the staging buffer is free for the next item's boxes
+    // the staging buffer is free for the next item's boxes; where the copy did
+    // not complete for some thread, all report and stop together (the columns'
+    // barriers below count on every thread)
+    if (__syncthreads_or(!ok)) {
+      if (threadIdx.x == 0) atomicOr(err, 2);
+      mbar_wait(&bar, parity);
+      return;
+    }
     const int next = item + gridDim.x;
     if (threadIdx.x == 0 && next < nitems) {
       // order the reads above (generic proxy) before the copy engine's
@@ -1822,11 +1825,7 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
 #pragma unroll
     for (int q = 0; q < 16; ++q) acc[q].x = acc[q].y = R(0);
     for (int k2 = 0; k2 < a.K; ++k2, parity ^= 1u) {
-      if (!mbar_wait(&bar, parity)) {  // the copy did not complete: report and stop
-        if (threadIdx.x == 0) atomicOr(err, 2);
-        mbar_wait(&bar, parity);
-        return;
-      }
+      const bool ok = mbar_wait(&bar, parity);
       C v[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
@@ -1836,7 +1835,13 @@ k_ucol_fwd_bulk(ColArgs a, int npl, int *err) {
         v[q].y = R(0);
         if (jv && keep) v[q] = stage[size_t(grp) * a.hseg + pos];
       }
-      __syncthreads();  // the staging buffer is free for the next segment
+      // the staging buffer is free for the next segment; all stop together where
+      // the copy did not complete (as k_ucol_bwd_tma)
+      if (__syncthreads_or(!ok)) {
+        if (threadIdx.x == 0) atomicOr(err, 2);
+        mbar_wait(&bar, parity);
+        return;
+      }
       if (threadIdx.x == 0) {
         int ni = item, nk = k2 + 1;
         if (nk == a.K) {

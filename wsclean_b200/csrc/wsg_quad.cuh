@@ -273,7 +273,7 @@ k_ucol_fwd_quad(ColArgs a, int npl, int *err) {
     if (item < nitems) issue(item, 0, 0);
   }
   __syncthreads();  // the barrier and the tables are in place
-  uint32_t parity = 0;
+  uint32_t parity = 0, open = 0;  // (open: the phase thread 0's last copy completes)
   bool ok = true;
   for (; item < nitems; item += gridDim.x) {
     const int lp = item / npairs, j0 = (item % npairs) * 2;
@@ -288,6 +288,7 @@ k_ucol_fwd_quad(ColArgs a, int npl, int *err) {
             if (waited != k2) {  // once a pass, at its first load
               waited = k2;
               ok = ok && mbar_wait(&bar, parity);
+              open = ok ? parity ^ 1u : open;
               parity ^= 1u;
             }
             const int m = Quad::freq(p, s), i = a.K * m + k2 + a.nx / 2;
@@ -315,7 +316,7 @@ k_ucol_fwd_quad(ColArgs a, int npl, int *err) {
     // a copy did not complete for some thread: all report and stop
     if (__syncthreads_or(!ok)) {
       if (threadIdx.x == 0) atomicOr(err, 2);
-      mbar_wait(&bar, parity);
+      mbar_wait(&bar, open);
       return;
     }
     int jx = j0 + a.joff;
