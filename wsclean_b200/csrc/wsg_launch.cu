@@ -151,19 +151,14 @@ struct ColKernels {
     const size_t smem = tws ? base + extra : base;
     auto *kern = tws ? k_ucol_bwd_tma<R, LOGM, true> : k_ucol_bwd_tma<R, LOGM, false>;
     smem_attr(kern, smem);
-    static int per_sm[2] = {-1, -1};  // resident CTAs per SM of each instantiation
-    if (per_sm[tws] < 0) {
-      int n = 0;
-      cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, ColCfg<R, M>::THREADS,
-                                                               smem),
-                 "occupancy");
-      per_sm[tws] = std::max(n, 1);
-    }
+    // (the shared memory depends on the band's height and on K)
+    const int per_sm =
+        resident_ctas(reinterpret_cast<const void *>(kern), ColCfg<R, M>::THREADS, smem);
     int dev = 0, nsm = 148;
     cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "attribute");
     const long long nitems = (long long)((a.ny + NB - 1) / NB) * npl;
-    const int grid = int(std::min<long long>(nitems, (long long)nsm * per_sm[tws]));
+    const int grid = int(std::min<long long>(nitems, (long long)nsm * per_sm));
     kern<<<grid, ColCfg<R, M>::THREADS, smem, st>>>(a, map, npl, err);
     cuda_check(cudaGetLastError(), "k_ucol_bwd_tma launch");
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
