@@ -262,6 +262,7 @@ void StreamGridder::copy_into(void *dst, const void *src, size_t bytes, PinnedBu
 // the scan and record kernels of each batch, from the finished grid of w.
 void StreamGridder::set_imaging_weights(const ImageWeightsGpu *w) {
   if (!w) {
+    flush_batch();  // (as below)
     iw_ = ImgW{};
     return;
   }
