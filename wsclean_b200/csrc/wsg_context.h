@@ -442,7 +442,10 @@ class ImageWeightsGpu {
   void get(double *grid, size_t *width, size_t *height, double *total);
   // the finished grid, for lookups while visibilities are gridded
   bool finished() const { return finished_; }
-  const double *grid_ptr() const { return reinterpret_cast<const double *>(grid_.p); }
+  const double *grid_ptr() const {
+    lent_ = true;
+    return reinterpret_cast<const double *>(grid_.p);
+  }
   WeightGrid geometry() const { return WeightGrid{int(W_), int(H_), psx_, psy_}; }
   int device() const { return cx_.device; }
 
@@ -454,6 +457,7 @@ class ImageWeightsGpu {
   size_t W_, H_;
   double psx_, psy_;
   bool as_taper_, finished_ = false;
+  mutable bool lent_ = false;  // grid_ptr() was given out
   DevBuf grid_, sums_, lambda_, in_, out_;
   std::shared_ptr<WeightSpare> spare_;
 };

@@ -38,7 +38,13 @@ ImageWeightsGpu::ImageWeightsGpu(Context &cx, int mode, double robust, size_t wi
 
 ImageWeightsGpu::~ImageWeightsGpu() {
   cudaSetDevice(cx_.device);
-  cudaStreamSynchronize(cx_.stream);
+  // (a gridding stream of another context, or of this one on another stream, may
+  // have lookups in flight, and the next object clears the grid: as cudaFree
+  // would, wait for the device)
+  if (lent_)
+    cudaDeviceSynchronize();
+  else
+    cudaStreamSynchronize(cx_.stream);
   {
     std::lock_guard<std::mutex> lk(spare_->mu);
     if (grid_.n > spare_->grid.n) {
