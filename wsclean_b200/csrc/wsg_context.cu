@@ -177,7 +177,7 @@ Context::~Context() {
   if (stream) cudaStreamSynchronize(stream);
   for (auto &kv : fft_plans) cufftDestroy(kv.second);
   for (auto *b : all_buffers()) b->release();
-  weight_spare->clear();
+  weight_spare.clear();
   for (auto &e : ev) cudaEventDestroy(e);
   for (cudaStream_t st : {cpy, d2h})
     if (st) {
@@ -237,7 +237,7 @@ void Context::release_buffers() {
   for (auto &kv : fft_plans) cufftDestroy(kv.second);
   fft_plans.clear();
   for (auto *b : all_buffers()) b->release();
-  weight_spare->clear();
+  weight_spare.clear();
   band_dirty = BandDirty{};
   bandd_zero = BandDirty{};
   invalidate_tables();

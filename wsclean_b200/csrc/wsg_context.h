@@ -7,7 +7,6 @@
 #include <chrono>
 #include <array>
 #include <map>
-#include <memory>
 #include <mutex>
 #include <utility>
 #include <tuple>
@@ -32,9 +31,8 @@ struct DevBuf {
 // The device buffers of an ImageWeights object that a context keeps for the
 // next one: allocating and freeing a 4096^2 image's grid took 0.3 to 10 ms, the
 // whole of gridding, finishing and looking up 8M weights takes 0.19.  At most
-// one set a context, freed with the context or by its release_buffers(); it is
-// shared so that an object outliving its context still hands its buffers to
-// someone who frees them.
+// one set a context, freed with it or by its release_buffers() (a context
+// outlives its objects: wsg_ctx_destroy refuses before).
 struct WeightSpare {
   std::mutex mu;
   DevBuf grid, sums, lambda;
@@ -204,7 +202,7 @@ class Context {
   void clear_band(void *band, size_t rows, size_t nv, size_t cs);
   void grid_fft(void *grid, const GridPlan &g, size_t P, size_t npl, int dir, bool dbl);
   DevBuf b_img, b_img2, b_acc, b_fftwork, b_out;
-  std::shared_ptr<WeightSpare> weight_spare = std::make_shared<WeightSpare>();
+  WeightSpare weight_spare;
 
  private:
   friend class Plan;
@@ -459,7 +457,6 @@ class ImageWeightsGpu {
   bool as_taper_, finished_ = false;
   mutable bool lent_ = false;  // grid_ptr() was given out
   DevBuf grid_, sums_, lambda_, in_, out_;
-  std::shared_ptr<WeightSpare> spare_;
 };
 
 // Allocation-free mixed-precision ms2dirty (scratch in a static device array).

@@ -19,14 +19,14 @@ ImageWeightsGpu::ImageWeightsGpu(Context &cx, int mode, double robust, size_t wi
   require(W_ >= 2 && H_ >= 2, "image-weight grid too small");
   CK(cudaSetDevice(cx_.device));
   const size_t bytes = W_ * (H_ / 2) * sizeof(double);
-  spare_ = cx_.weight_spare;
   {
+    WeightSpare &spare = cx_.weight_spare;
     // the last object's buffers, unless they are far too large
-    std::lock_guard<std::mutex> lk(spare_->mu);
-    if (spare_->grid.n >= bytes && spare_->grid.n / 4 <= bytes) {
-      std::swap(grid_, spare_->grid);
-      std::swap(sums_, spare_->sums);
-      std::swap(lambda_, spare_->lambda);
+    std::lock_guard<std::mutex> lk(spare.mu);
+    if (spare.grid.n >= bytes && spare.grid.n / 4 <= bytes) {
+      std::swap(grid_, spare.grid);
+      std::swap(sums_, spare.sums);
+      std::swap(lambda_, spare.lambda);
     }
   }
   grid_.ensure(bytes);
@@ -46,11 +46,12 @@ ImageWeightsGpu::~ImageWeightsGpu() {
   else
     cudaStreamSynchronize(cx_.stream);
   {
-    std::lock_guard<std::mutex> lk(spare_->mu);
-    if (grid_.n > spare_->grid.n) {
-      std::swap(grid_, spare_->grid);
-      std::swap(sums_, spare_->sums);
-      std::swap(lambda_, spare_->lambda);
+    WeightSpare &spare = cx_.weight_spare;
+    std::lock_guard<std::mutex> lk(spare.mu);
+    if (grid_.n > spare.grid.n) {
+      std::swap(grid_, spare.grid);
+      std::swap(sums_, spare.sums);
+      std::swap(lambda_, spare.lambda);
     }
   }
   for (DevBuf *b : {&grid_, &sums_, &lambda_, &in_, &out_}) b->release();
