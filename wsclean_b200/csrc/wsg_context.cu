@@ -215,7 +215,7 @@ void Context::synchronize() {
   CK(cudaStreamSynchronize(d2h));
   if (err_pending) {
     err_pending = false;
-    check_device_error(reinterpret_cast<const int *>(reinterpret_cast<char *>(b_small.p) + 3072));
+    check_device_error(small_int(kOffErr));
   }
   for (int *w : plan_err) {
     int h = 0;
@@ -338,7 +338,8 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
   // reads on the copy stream: its read-back then waits for this call's
   // copies only, not for earlier calls' kernels on the main stream
   cudaStream_t sst = scan_st ? scan_st : stream;
-  ScanOut *d_scan = reinterpret_cast<ScanOut *>(b_small.ensure(4096));
+  static_assert(sizeof(ScanOut) <= kOffChunks, "layout of b_small");
+  ScanOut *d_scan = reinterpret_cast<ScanOut *>(b_small.ensure(kSmallBytes));
   // on the main stream, with no error word to keep (a stream's stays from batch
   // to batch), one upload sets the
   // initial statistics, clears the counters and the error word and brings f/c
@@ -350,7 +351,7 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
   double *d_fovc = reinterpret_cast<double *>(
       one ? static_cast<char *>(b_small.p) + kOffFovc
           : static_cast<char *>(fbuf.ensure(a.nchan * sizeof(double))));
-  const size_t small_bytes = std::max<size_t>(4096, sizeof(ScanOut) + a.nchan * sizeof(double));
+  const size_t small_bytes = std::max<size_t>(kSmallBytes, sizeof(ScanOut) + a.nchan * sizeof(double));
   if (h_small_cap < small_bytes) {
     if (h_small) CK(cudaFreeHost(h_small));
     h_small = nullptr;
@@ -493,7 +494,7 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
   const int chunk = gp.batch ? chunk_max
                              : int(std::min<size_t>(chunk_max, std::max<size_t>(
                                        chunk_min, gp.nvis / (4 * size_t(num_sms)))));
-  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
+  int *d_nch = small_int(kOffChunks);
 
   // keys (unless the scan wrote them for this grid) + sort
   if (nvis_tot <= kSmallMax && !gp.wide_keys) {
@@ -845,9 +846,9 @@ bool Context::grid_core(const wsg_args &a, const Staged &s, double *img, bool ac
   if (!gp.ucufft) ca = make_col(gp, P, u_tables(gp, dbl), bandf, H);
   const void *twv = gp.vprune ? v_tables(gp) : nullptr;
   const long Lv = band_v_halfwidth(gp);
-  int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
-  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
-  int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
+  int *counter = small_int(kOffCounter);
+  int *d_nch = small_int(kOffChunks);
+  int *d_err = small_int(kOffErr);
   if (!err_pending && !small_zeroed)
     CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));  // sticky while pipelined
   GridArgs ga{};
@@ -986,9 +987,9 @@ void Context::degrid_core(const wsg_args &a, const Staged &s, const double *img,
   ColArgs ca{};
   if (!gp.ucufft) ca = make_col(gp, P, u_tables(gp, dbl), bandi, H);
   const void *twv = gp.vprune ? v_tables(gp) : nullptr;
-  int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 2048);
-  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 1024);
-  int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(b_small.p) + 3072);
+  int *counter = small_int(kOffCounter);
+  int *d_nch = small_int(kOffChunks);
+  int *d_err = small_int(kOffErr);
   if (!err_pending && !small_zeroed)
     CK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));  // sticky while pipelined
   GridArgs ga{};

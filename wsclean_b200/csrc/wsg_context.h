@@ -169,7 +169,13 @@ class Context {
   // layout of b_small (bytes): the scan's statistics, then the chunk count,
   // the chunk counter, the error word, f/c of up to kSmallChan channels
   static constexpr size_t kOffChunks = 1024, kOffCounter = 2048, kOffErr = 3072, kOffFovc = 3328;
-  static constexpr size_t kSmallChan = (4096 - kOffFovc) / sizeof(double);
+  static constexpr size_t kSmallBytes = 4096, kSmallChan = (kSmallBytes - kOffFovc) / sizeof(double);
+  static_assert(kOffChunks < kOffCounter && kOffCounter < kOffErr &&
+                    kOffErr + sizeof(int) <= kOffFovc && kOffFovc < kSmallBytes,
+                "prepare()'s upload clears everything before f/c");
+  int *small_int(size_t off) {
+    return reinterpret_cast<int *>(static_cast<char *>(b_small.p) + off);
+  }
   // prepare() zeroed the counter and the error word with its upload
   bool small_zeroed = false;
   void finish_call(const wsg_args &a, Slot &sl, cudaStream_t last);

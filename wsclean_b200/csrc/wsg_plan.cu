@@ -171,8 +171,8 @@ void Plan::build(const std::vector<wsg_job> &js) {
     require(gp.T == T_ && gp.kernel.W == W_, "internal: jobs must share kernel and tile");
     pj.nrec = gp.nvis;
     int nch_j = 0;
-    CK(cudaMemcpyAsync(&nch_j, reinterpret_cast<char *>(cx_.b_small.p) + 1024, sizeof(int),
-                       cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&nch_j, cx_.small_int(Context::kOffChunks), sizeof(int), cudaMemcpyDeviceToHost,
+                       st));
     CK(cudaStreamSynchronize(st));
     pj.rec_off = nrec_;
     CK(cudaMemcpyAsync(static_cast<char *>(rec_.p) + nrec_ * sizeof(Rec), cx_.b_rec.p,

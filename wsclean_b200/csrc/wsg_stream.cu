@@ -214,9 +214,9 @@ void StreamGridder::add_t(const Staged &s, size_t nrows) {
   GridPlan g = gp_;
   if (!cx_.prepare<R>(ac, s, true, nullptr, g)) return;
   cudaStream_t st = cx_.stream;
-  int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 2048);
-  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 1024);
-  int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 3072);
+  int *counter = cx_.small_int(Context::kOffCounter);
+  int *d_nch = cx_.small_int(Context::kOffChunks);
+  int *d_err = cx_.small_int(Context::kOffErr);
   if (!err_armed_) {  // read back and cleared by finish()
     CK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
     err_armed_ = true;
@@ -392,7 +392,7 @@ void StreamGridder::finish_t(void *dirty, int accumulate) {
   // planes per pass: as many planes of u-transformed rows as H holds (all of
   // them with the whole-grid layout)
   const size_t P = g.ucufft ? g.nplanes : std::max<size_t>(1, H_.n / row_plane_bytes());
-  int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 3072);
+  int *d_err = cx_.small_int(Context::kOffErr);
   if (!err_armed_) {
     CK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
     err_armed_ = true;
@@ -448,7 +448,8 @@ void StreamGridder::predict_begin_t(const void *img, int in_f32) {
   const GridPlan &g = gp_;
   cudaStream_t st = cx_.stream;
   const size_t cs = 2 * sizeof(R);
-  int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.ensure(4096)) + 3072);
+  cx_.b_small.ensure(Context::kSmallBytes);
+  int *d_err = cx_.small_int(Context::kOffErr);
   CK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
   // (the pruned v transform writes every band entry)
   if (!g.vprune) CK(cudaMemsetAsync(band_.p, 0, band_.n, st));
@@ -518,9 +519,9 @@ void StreamGridder::predict_t(const Staged &s, size_t nrows, void *vis_dev) {
   GridPlan g = gp_;
   if (!cx_.prepare<R>(ac, s, false, vis_dev, g)) return;
   cudaStream_t st = cx_.stream;
-  int *counter = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 2048);
-  int *d_nch = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 1024);
-  int *d_err = reinterpret_cast<int *>(reinterpret_cast<char *>(cx_.b_small.p) + 3072);
+  int *counter = cx_.small_int(Context::kOffCounter);
+  int *d_nch = cx_.small_int(Context::kOffChunks);
+  int *d_err = cx_.small_int(Context::kOffErr);
   CK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
   CK(cudaMemsetAsync(counter, 0, sizeof(int), st));
   GridArgs ga{};
