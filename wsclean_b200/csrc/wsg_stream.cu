@@ -602,7 +602,7 @@ void StreamGridder::stats(wsg_stats &o) const {
   o.dw = g.dw;
   o.nshift = g.nshift;
   o.precision = g.fp32 ? WSG_PREC_MIXED : WSG_PREC_FP64;
-  o.device_bytes = band_.n + H_.n + img_.n + fftwork_.n;
+  o.device_bytes = band_.n + hv_.n + H_.n + img_.n + fftwork_.n;
   o.kernel_launches = g_kernel_launches.load();
 }
 
