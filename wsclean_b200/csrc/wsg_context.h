@@ -254,7 +254,7 @@ class Context {
   PlanesMemo planes_memo[2];  // degridding, gridding
   // last grid plan per direction, keyed by the arguments and data statistics
   struct GridMemo {
-    std::array<double, 22> key{};
+    std::array<double, 23> key{};
     GridPlan plan;
     bool valid = false;
   };
