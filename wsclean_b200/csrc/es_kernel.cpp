@@ -461,7 +461,7 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
   // 1e-4); elsewhere the library transforms whole rows.  The w planes keep the
   // spacing of the library's height.
   g.vprune = false;
-  if (g.fp32 && !pow2_v && !g.ucufft) {
+  if (g.fp32 && !pow2_v && !g.ucufft && !g.whole_rows) {
     const double vmax_px = g.vmax * g.py;
     auto width = [&](size_t nv) { return 2.0 * std::ceil(vmax_px * double(nv) + 0.5 * W + 2.0) + 1.0; };
     size_t nv = 0;
@@ -695,6 +695,11 @@ size_t plan_bytes(const GridPlan &g, size_t planes, bool gridding) {
   // both directions keep the grid and its v transform apart, plus the
   // u-transformed rows
   return planes * cs * (2 * g.band_rows * g.nv + g.ny * g.hrow());
+}
+
+size_t resident_bytes(const GridPlan &g) {
+  const size_t cs = g.fp32 ? 8 : 16;
+  return cs * g.nplanes * g.band_rows * (g.vprune ? g.nvs() + g.ncol() : g.nv);
 }
 
 }  // namespace wsg

@@ -254,7 +254,7 @@ class Context {
   PlanesMemo planes_memo[2];  // degridding, gridding
   // last grid plan per direction, keyed by the arguments and data statistics
   struct GridMemo {
-    std::array<double, 23> key{};
+    std::array<double, 24> key{};
     GridPlan plan;
     bool valid = false;
   };
@@ -337,6 +337,7 @@ class Plan {
   std::vector<PlanJob> jobs_;
   DevBuf rec_, chunks_, chunk_job_, jobgeom_, band_, H_, hv_, img_, cf_, tw_, small_, fftwork_;
   size_t nrec_ = 0, band_total_ = 0, max_npix_ = 0;
+  bool whole_rows_ = false;  // the jobs' GridPlan::whole_rows
   int nchunks_ = 0;
   std::vector<unsigned char> kernel_;  // DevKernel<R> bytes
   std::vector<unsigned char> geom_;    // DevGeom of the first job (kernel, tile: shared)

@@ -44,6 +44,8 @@ void cufft_check(cufftResult r, const char *what);
 int env_int(const char *name, int dflt);
 // Bin tile edge asked of the planner.
 int default_tile(bool fp32);
+// Free device memory; WSG_FREE_MB (a test and debugging limit) lowers it.
+size_t free_device_bytes();
 
 // ------------------------------------------------------------- planning
 

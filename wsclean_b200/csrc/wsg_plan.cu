@@ -73,6 +73,9 @@ void Plan::build(const std::vector<wsg_job> &js) {
   const size_t nchan = a_.nchan, nrows = a_.nrows;
   cudaStream_t st = cx_.stream;
   const int tile = default_tile(sizeof(R) == 4);
+  const size_t spare = free_device_bytes() / 16;  // (see below)
+  nrec_ = band_total_ = max_npix_ = 0;
+  nchunks_ = 0;
 
   // coordinates on the device (kept only while building)
   Staged s;
@@ -154,6 +157,7 @@ void Plan::build(const std::vector<wsg_job> &js) {
     gp.force_W = forceW;
     gp.force_sigma = forceS;
     gp.batch = jobs_.size() > 1;
+    gp.whole_rows = whole_rows_;
     const bool any = cx_.prepare<R>(aj, sj, false, nullptr, gp);
     if (forceW == 0 && any) {  // the largest job with active visibilities
       forceW = gp.kernel.W;
@@ -219,6 +223,26 @@ void Plan::build(const std::vector<wsg_job> &js) {
     max_npix_ = std::max(max_npix_, gp.nx * gp.ny);
   }
   require(nrec_ > 0, "no active visibilities in any job");
+  // the pruned form's second array (one for all jobs) may take more memory than
+  // the columns it leaves out: up to 1/16 of what is free, as in a stream
+  if (!whole_rows_) {
+    size_t pruned = band_total_, whole = 0, second = 0;
+    for (const auto &pj : jobs_)
+      if (pj.nrec > 0) second = std::max(second, resident_bytes(pj.gp) - pj.band_bytes);
+    if (second > 0 && pruned + second > spare) {
+      for (const auto &pj : jobs_) {
+        if (pj.nrec == 0) continue;
+        GridPlan w = pj.gp;
+        w.whole_rows = true;
+        choose_grid(w, a_.sigma_min, a_.sigma_max, tile);
+        whole += align256(resident_bytes(w));
+      }
+      if (pruned + second > whole + spare) {
+        whole_rows_ = true;
+        return build<R>(js);
+      }
+    }
+  }
   CK(cudaMemcpyAsync(small_.p, &nchunks_, sizeof(int), cudaMemcpyHostToDevice, st));
 
   size_t hmax = 0, work = 0, hvmax = 0;
