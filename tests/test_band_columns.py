@@ -17,7 +17,8 @@ PROGRAM = r'''
 int main() {
   long wrong = 0, pruned = 0, both = 0, whole = 0;
   for (double eps : {1e-3, 1e-4, 1e-5})
-    for (int ny : {64, 128, 160, 170, 250, 340, 512, 640, 680, 1024, 2048})
+    for (int ny : {64, 128, 136, 150, 160, 170, 180, 250, 276, 300, 340, 360, 512, 560, 640, 680, 720,
+                   1024, 1118, 2048})
       for (double vpx : {0.1, 0.3, 0.4, 0.46, 0.465, 0.47, 0.48, 0.488, 0.492, 0.494, 0.498}) {
         wsg::GridPlan g;
         g.nx = 64;
@@ -67,5 +68,5 @@ def test_columns_of_every_tile(tmp_path):
                     str(src), os.path.join(CSRC, "es_kernel.cpp"), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout
     wrong, pruned, both, whole = (int(x) for x in out.split())
-    assert pruned > 50 and both > 0 and whole > 0, out
+    assert pruned > 50 and both > 20 and whole > 0, out
     assert wrong == 0, out

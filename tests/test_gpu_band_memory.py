@@ -43,7 +43,7 @@ def test_whole_rows_where_memory_is_short(kind, monkeypatch):
     import torch
     import oracle as O
     from wsclean_b200.gridder import Plan, Stream, data_extent
-    nx, ny, px, v, eps = 128, 512, 1e-4, 0.45, 1e-5
+    nx, ny, px, v, eps = 128, 600, 1e-4, 0.45, 1e-5
     uvw, vis = _data(3000, px, v)
     ref = O.dft_ms2dirty(uvw, FREQ, vis, nx, ny, px, px, negate_v=True, divide_by_n=False)
     dev = torch.device("cuda", 0)

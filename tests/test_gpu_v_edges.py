@@ -14,7 +14,8 @@ FREQ = np.array([1.5e8])
 LAM = 299792458.0 / FREQ[0]
 NX, PX = 64, 0.08 / 256
 CASES = [(64, 1e-5, 0.47), (128, 1e-5, 0.47), (160, 1e-5, 0.47), (512, 1e-5, 0.492),
-         (160, 1e-4, 0.47), (640, 1e-3, 0.494)]
+         (160, 1e-4, 0.47), (640, 1e-3, 0.494), (196, 1e-3, 0.47), (180, 1e-4, 0.46),
+         (720, 1e-4, 0.488), (322, 1e-5, 0.47), (658, 1e-5, 0.488)]
 
 
 def _data(ny, vmax_px):
@@ -45,7 +46,7 @@ def test_call(ny, eps, vmax_px):
     ctx.close()
 
 
-@pytest.mark.parametrize("ny,eps,vmax_px", CASES[:1] + CASES[3:4])
+@pytest.mark.parametrize("ny,eps,vmax_px", CASES[:1] + CASES[2:4] + CASES[-1:])
 def test_plan_and_stream(ny, eps, vmax_px):
     import torch
     uvw, vis, img, ref, mref = _data(ny, vmax_px)

@@ -454,12 +454,19 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
   g.ofactor = std::min(double(g.nu) / g.nx, double(g.nv) / g.ny);
   const int W = bestk.W;
   // The mixed form's pruned v transform: nv = Kv * 2^m.  The grid height the
-  // library transform would take is kept where it has that form.  A different
-  // height changes the image by about the kernel's aliasing error, so another
-  // one (the next with that form) is taken only where that error is at most
-  // 1e-5 (measured: 1e-6 to 2e-6 of the image at epsilon 1e-5, but 2e-5 at
-  // 1e-4); elsewhere the library transforms whole rows.  The w planes keep the
-  // spacing of the library's height.
+  // library transform would take is kept where it has that form.  Another one
+  // (the next with that form) moves the image by about the kernel's aliasing
+  // error (1e-6 to 2e-6 of it at epsilon 1e-5, 2e-5 at 1e-4) and makes every
+  // band and bin taller, so it is taken only where that error is at most 1e-5
+  // and the pruned form is the faster one: at most 1.2 times as tall with stored
+  // columns of at most 0.6 of the library's row, 1.1 times and 0.8, or in grids of
+  // up to 1024 rows, where launches count, 1.5 times.  Over 945 geometries (400^2
+  // to 8400^2, 0.06 to 1.5 visibilities a pixel, heights up to 1.5 times) pruned /
+  // whole rows are 0.97 (grid) and 0.99 (predict) inside these limits, 0.965 in
+  // total time; outside 1.03 and 1.05, 1.06 in total and 1.16 at the 95th
+  // percentile (3148^2 at 0.42 cycles a pixel, 4608 -> 8192 rows: 10.1 -> 14.5 ms).
+  // Inside: 8192^2 stream, 14000 -> 16384, 69.2 -> 58.1 ms.
+  // The w planes keep the spacing of the library's height.
   g.vprune = false;
   if (g.fp32 && !pow2_v && !g.ucufft && !g.whole_rows) {
     const double vmax_px = g.vmax * g.py;
@@ -474,8 +481,15 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
         kk = int(nv / M);
       }
     }
-    if (nv == 0 && g.kernel.err <= 1.05e-5)
-      if (!pick_nu(std::max(64.0, g.ny * bestk.sigma), vmax_px, W, nv, lm, kk)) nv = 0;
+    if (nv == 0 && g.kernel.err <= 1.05e-5) {
+      const double nl = double(g.nv);
+      auto pays = [&](double taller, double stored) {
+        return double(nv) <= taller * nl && width(nv) <= stored * nl;
+      };
+      if (!pick_nu(std::max(64.0, g.ny * bestk.sigma), vmax_px, W, nv, lm, kk) ||
+          !(pays(1.1, 0.8) || pays(1.2, 0.6) || (nv <= 1024 && pays(1.5, 1.5))))
+        nv = 0;
+    }
     if (nv != 0 && nv < 65000 && width(nv) < double(nv)) {
       g.vprune = true;
       g.nv = nv;
