@@ -1,8 +1,9 @@
 """The height of the pruned mixed form, on the host: the library's height where
 it has the form, else a taller one only within the limits where it measured
-faster -- at most 1.2 times as tall with the stored columns at most 0.6 of the
-library's row, 1.1 times and 0.8, or 1.5 times up to 1024 rows -- so that no
-call pays for a much taller grid."""
+faster, so that no call pays for a much taller grid.  Calls: at most 1.2 times as
+tall with the stored columns at most 0.6 of the library's row, or 1.1 times and
+0.8; grids that plans and streams keep: 1.35 times and 0.7; both 1.5 times up to
+1024 rows."""
 import os
 import subprocess
 
@@ -31,7 +32,8 @@ PROGRAM = r'''
 
 int main() {
   long higher = 0, natural = 0, whole = 0, wrong = 0;
-  for (double eps : {1e-4, 1e-5})
+  for (bool resident : {false, true})
+   for (double eps : {1e-4, 1e-5})
     for (int n = 200; n < 9000; n += 2 * (1 + n / 40))
       for (double v : {0.05, 0.12, 0.2, 0.28, 0.36, 0.45}) {
         wsg::GridPlan g;
@@ -43,6 +45,7 @@ int main() {
         g.nvis = 1000000;
         g.wmax_d = 200;
         g.umax = g.vmax = v / g.px;
+        g.resident = resident;
         wsg::GridPlan w = g;
         w.whole_rows = true;
         wsg::choose_grid(g, 1.1, 2.0, 24);
@@ -56,7 +59,9 @@ int main() {
         } else {
           ++higher;
           const double taller = double(g.nv) / w.nv, stored = (double(g.nvs()) - 1) / w.nv;
-          const bool pays = (taller <= 1.1 && stored <= 0.8) || (taller <= 1.2 && stored <= 0.6) ||
+          const bool pays = (taller <= 1.1 && stored <= 0.8) ||
+                            (resident ? taller <= 1.35 && stored <= 0.7
+                                      : taller <= 1.2 && stored <= 0.6) ||
                             (g.nv <= 1024 && taller <= 1.5);
           if (!pays || g.kernel.err > 1.05e-5) ++wrong;
         }

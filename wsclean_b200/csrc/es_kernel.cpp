@@ -465,7 +465,10 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
   // whole rows are 0.97 (grid) and 0.99 (predict) inside these limits, 0.965 in
   // total time; outside 1.03 and 1.05, 1.06 in total and 1.16 at the 95th
   // percentile (3148^2 at 0.42 cycles a pixel, 4608 -> 8192 rows: 10.1 -> 14.5 ms).
-  // Inside: 8192^2 stream, 14000 -> 16384, 69.2 -> 58.1 ms.
+  // Plans and streams clear the whole grid, a call the columns it wrote, so that
+  // the former go to 1.35 times and 0.7: 981 streams, 0.95 inside (0.97 between
+  // the two limits), 0.99 outside; 8192^2, 14000 -> 16384: 69.2 -> 58.1 ms, 12288
+  // -> 16384: 62.0 -> 60.0.
   // The w planes keep the spacing of the library's height.
   g.vprune = false;
   if (g.fp32 && !pow2_v && !g.ucufft && !g.whole_rows) {
@@ -487,7 +490,8 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
         return double(nv) <= taller * nl && width(nv) <= stored * nl;
       };
       if (!pick_nu(std::max(64.0, g.ny * bestk.sigma), vmax_px, W, nv, lm, kk) ||
-          !(pays(1.1, 0.8) || pays(1.2, 0.6) || (nv <= 1024 && pays(1.5, 1.5))))
+          !(pays(1.1, 0.8) || (g.resident ? pays(1.35, 0.7) : pays(1.2, 0.6)) ||
+            (nv <= 1024 && pays(1.5, 1.5))))
         nv = 0;
     }
     if (nv != 0 && nv < 65000 && width(nv) < double(nv)) {
@@ -709,6 +713,11 @@ size_t plan_bytes(const GridPlan &g, size_t planes, bool gridding) {
   // both directions keep the grid and its v transform apart, plus the
   // u-transformed rows
   return planes * cs * (2 * g.band_rows * g.nv + g.ny * g.hrow());
+}
+
+size_t whole_rows_bytes(const GridPlan &g) {
+  const size_t cs = g.fp32 ? 8 : 16;
+  return cs * g.nplanes * g.band_rows * size_t(double(g.ny) * g.kernel.sigma);
 }
 
 size_t resident_bytes(const GridPlan &g) {

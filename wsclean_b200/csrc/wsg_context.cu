@@ -472,12 +472,12 @@ bool Context::prepare(const wsg_args &a, const Staged &s, bool gridding, void *v
     }
     // the same data statistics and arguments give the same plan: repeated
     // calls reuse the previous one of their direction
-    const std::array<double, 24> key{
+    const std::array<double, 25> key{
         double(gp.nx), double(gp.ny), gp.px, gp.py, gp.eps, double(gp.do_w), double(gp.fp32),
         double(gp.negate_v), double(gp.divide_by_n), gp.lshift, gp.mshift, double(gp.nvis),
         gp.wmin_d, gp.wmax_d, gp.umax, gp.vmax, double(gp.force_W), gp.force_sigma,
         a.sigma_min, a.sigma_max, double(tile), double(gp.gridding), double(gp.batch),
-        double(gp.whole_rows)};
+        double(gp.resident), double(gp.whole_rows)};
     GridMemo &gm = grid_memo[gridding ? 1 : 0];
     if (gm.valid && gm.key == key) {
       gp = gm.plan;

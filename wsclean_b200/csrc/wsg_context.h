@@ -254,7 +254,7 @@ class Context {
   PlanesMemo planes_memo[2];  // degridding, gridding
   // last grid plan per direction, keyed by the arguments and data statistics
   struct GridMemo {
-    std::array<double, 24> key{};
+    std::array<double, 25> key{};
     GridPlan plan;
     bool valid = false;
   };

@@ -186,6 +186,8 @@ struct GridPlan {
   double force_sigma = 0;
   // a batch plan's job: its chunks share their launches with the other jobs'
   bool batch = false;
+  // plans and streams: the band grid holds all planes, and is cleared whole
+  bool resident = false;
   // whole band rows in any case (plans and streams short of memory)
   bool whole_rows = false;
   // streams: the grid was planned from a declared data extent; chunks are
@@ -287,5 +289,7 @@ size_t plan_bytes(const GridPlan &g, size_t planes, bool gridding);
 // Bytes of the band arrays of a grid that keeps all its planes (plans,
 // streams): the band grid and, in the pruned form, the rows transformed along v.
 size_t resident_bytes(const GridPlan &g);
+// ... and about what whole rows of the library's height would take.
+size_t whole_rows_bytes(const GridPlan &g);
 
 }  // namespace wsg

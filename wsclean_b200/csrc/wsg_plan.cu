@@ -157,6 +157,7 @@ void Plan::build(const std::vector<wsg_job> &js) {
     gp.force_W = forceW;
     gp.force_sigma = forceS;
     gp.batch = jobs_.size() > 1;
+    gp.resident = true;
     gp.whole_rows = whole_rows_;
     const bool any = cx_.prepare<R>(aj, sj, false, nullptr, gp);
     if (forceW == 0 && any) {  // the largest job with active visibilities
@@ -226,21 +227,15 @@ void Plan::build(const std::vector<wsg_job> &js) {
   // the pruned form's second array (one for all jobs) may take more memory than
   // the columns it leaves out: up to 1/16 of what is free, as in a stream
   if (!whole_rows_) {
-    size_t pruned = band_total_, whole = 0, second = 0;
-    for (const auto &pj : jobs_)
-      if (pj.nrec > 0) second = std::max(second, resident_bytes(pj.gp) - pj.band_bytes);
-    if (second > 0 && pruned + second > spare) {
-      for (const auto &pj : jobs_) {
-        if (pj.nrec == 0) continue;
-        GridPlan w = pj.gp;
-        w.whole_rows = true;
-        choose_grid(w, a_.sigma_min, a_.sigma_max, tile);
-        whole += align256(resident_bytes(w));
-      }
-      if (pruned + second > whole + spare) {
-        whole_rows_ = true;
-        return build<R>(js);
-      }
+    size_t whole = 0, second = 0;
+    for (const auto &pj : jobs_) {
+      if (pj.nrec == 0) continue;
+      whole += pj.gp.vprune ? whole_rows_bytes(pj.gp) : pj.band_bytes;
+      second = std::max(second, resident_bytes(pj.gp) - pj.band_bytes);
+    }
+    if (second > 0 && band_total_ + second > whole + spare) {
+      whole_rows_ = true;
+      return build<R>(js);
     }
   }
   CK(cudaMemcpyAsync(small_.p, &nchunks_, sizeof(int), cudaMemcpyHostToDevice, st));

@@ -64,17 +64,15 @@ StreamGridder::StreamGridder(Context &cx, const wsg_args &a, double wmin, double
   g.wmax_d = wmax;
   g.umax = umax;
   g.vmax = vmax;
+  g.resident = true;
   choose_grid(g, a.sigma_min, a.sigma_max, default_tile(!dbl_));
   // the pruned form's two arrays take up to 1.6 times the memory of whole rows
   // transformed in place: not more than 1/16 of what is free goes to that
   // (8192^2, 13 planes of 8.0k rows: 12.0 GB against 11.7, and 58 ms a pass
   // against 69)
-  const size_t spare = free_device_bytes() / 16;
-  if (g.vprune && resident_bytes(g) > spare) {
-    GridPlan w = g;
-    w.whole_rows = true;
-    choose_grid(w, a.sigma_min, a.sigma_max, default_tile(!dbl_));
-    if (resident_bytes(g) > resident_bytes(w) + spare) g = w;
+  if (g.vprune && resident_bytes(g) > whole_rows_bytes(g) + free_device_bytes() / 16) {
+    g.whole_rows = true;
+    choose_grid(g, a.sigma_min, a.sigma_max, default_tile(!dbl_));
   }
   g.fixed = true;
   const size_t cs = dbl_ ? 16 : 8;
