@@ -41,10 +41,13 @@ inline void require(bool ok, const std::string &msg) {
 // footprints of both ends of the band, whose columns are the row's last and
 // first ones.
 constexpr int band_col(int v, int Lv, int nv) { return v + Lv - (v + Lv >= nv ? nv : 0); }
-// ... of the cell c (< nv) further on, or -1 outside the row.
+// ... of the cell c further on, or -1 outside the row.  (A line ends less than a
+// kernel past nv, but on small grids it may start below 0 and pass nv twice: the
+// smallest of the three candidates, the wrong ones being huge as unsigned.)
 constexpr int band_col_next(int first, int c, int nv, int nvs) {
-  const int v = first + c - (first + c >= nv ? nv : 0);
-  return v < nvs ? v : -1;
+  const unsigned v = unsigned(first) + unsigned(c), n = unsigned(nv);
+  const unsigned v1 = v < v - n ? v : v - n, v2 = v1 < v - 2 * n ? v1 : v - 2 * n;
+  return v2 < unsigned(nvs) ? int(v2) : -1;
 }
 
 // One row of the generated ES kernel table.
