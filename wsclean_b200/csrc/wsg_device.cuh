@@ -1123,7 +1123,8 @@ k_ucol_bwd(ColArgs a) {
 // twiddles are loaded once per CTA instead of once per column group.  The
 // transforms run in place in one buffer per column (the staging buffer
 // takes the place of the second one).
-// Bound by issue (the FFT's arithmetic and shared-memory accesses), not DRAM:
+// Bound by latency at 16 warps an SM (127 registers): issue slots 59 % busy, the
+// shared-memory pipe 69 %, DRAM 36 %.
 // 4096^2, M = 2048, K = 3, 14 planes: 0.99 ms; with barriers of one column's
 // threads instead of the CTA's 0.91, with the twist factors multiplied out
 // (fill_twist) 0.87.

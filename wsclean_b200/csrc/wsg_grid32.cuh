@@ -7,8 +7,8 @@
 // q + 32 k of the footprint and their W cells along v, which stay in registers
 // while the origin repeats.
 //
-// What bounds it: issue slots (60-63% busy), then fixed-latency waits; DRAM is
-// at 4-6%.  So
+// What bounds it: latency at 16 warps an SM (fixed-latency waits first), with issue
+// slots 59-64% and the shared-memory pipe 44-51% busy; DRAM is at 5-6%.  So
 //  * cells are kept as pairs along v, real and imaginary parts apart: the
 //    kernel values along v are pairs as loaded, and one two-lane multiply-add
 //    serves two cells with no register moves (pairs of (re, im) needed every
@@ -23,8 +23,8 @@
 // Two CTAs an SM, 128 registers a thread: 3 x 8 and 2 x 12 warps an SM (80
 // registers) spill and were 5-10% slower; two tiles an SM also leave room for
 // 24 x 24 cells (20 x 20: 6% slower).  8.1M visibilities at 4096^2, W = 8:
-// spread 1.595 -> 1.046 ms, interpolation 1.310 -> 1.21 ms; 3.3M at 2048^2,
-// W = 7: 0.720 -> 0.530, 0.611 -> 0.580 ms.
+// spread 1.595 -> 1.046 ms, interpolation 1.310 -> 1.236 ms; 3.3M at 2048^2,
+// W = 7: 0.720 -> 0.562, 0.611 -> 0.606 ms.
 #pragma once
 
 #include "wsg_tile.cuh"
