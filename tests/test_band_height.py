@@ -2,8 +2,9 @@
 it has the form, else a taller one only within the limits where it measured
 faster, so that no call pays for a much taller grid.  Calls: at most 1.2 times as
 tall with the stored columns at most 0.6 of the library's row, or 1.1 times and
-0.8; grids that plans and streams keep: 1.35 times and 0.7; both 1.5 times up to
-1024 rows."""
+0.8; grids that plans and streams keep: 1.5 times and 0.7, or 1.2 times and 0.8;
+any height up to 1024 rows.
+"""
 import os
 import subprocess
 
@@ -59,10 +60,9 @@ int main() {
         } else {
           ++higher;
           const double taller = double(g.nv) / w.nv, stored = (double(g.nvs()) - 1) / w.nv;
-          const bool pays = (taller <= 1.1 && stored <= 0.8) ||
-                            (resident ? taller <= 1.35 && stored <= 0.7
-                                      : taller <= 1.2 && stored <= 0.6) ||
-                            (g.nv <= 1024 && taller <= 1.5);
+          auto within = [&](double t, double c) { return taller <= t && stored <= c; };
+          const bool pays = g.nv <= 1024 || (resident ? within(1.5, 0.7) || within(1.2, 0.8)
+                                                      : within(1.2, 0.6) || within(1.1, 0.8));
           if (!pays || g.kernel.err > 1.05e-5) ++wrong;
         }
       }

@@ -458,17 +458,16 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
   // (the next with that form) moves the image by about the kernel's aliasing
   // error (1e-6 to 2e-6 of it at epsilon 1e-5, 2e-5 at 1e-4) and makes every
   // band and bin taller, so it is taken only where that error is at most 1e-5
-  // and the pruned form is the faster one: at most 1.2 times as tall with stored
-  // columns of at most 0.6 of the library's row, 1.1 times and 0.8, or in grids of
-  // up to 1024 rows, where launches count, 1.5 times.  Over 945 geometries (400^2
-  // to 8400^2, 0.06 to 1.5 visibilities a pixel, heights up to 1.5 times) pruned /
-  // whole rows are 0.97 (grid) and 0.99 (predict) inside these limits, 0.965 in
-  // total time; outside 1.03 and 1.05, 1.06 in total and 1.16 at the 95th
-  // percentile (3148^2 at 0.42 cycles a pixel, 4608 -> 8192 rows: 10.1 -> 14.5 ms).
-  // Plans and streams clear the whole grid, a call the columns it wrote, so that
-  // the former go to 1.35 times and 0.7: 981 streams, 0.95 inside (0.97 between
-  // the two limits), 0.99 outside; 8192^2, 14000 -> 16384: 69.2 -> 58.1 ms, 12288
-  // -> 16384: 62.0 -> 60.0.
+  // and the pruned form is the faster one.  Calls: at most 1.2 times as tall with
+  // stored columns of at most 0.6 of the library's row, or 1.1 times and 0.8.  Over
+  // 945 geometries (400^2 to 8400^2, 0.06 to 1.5 visibilities a pixel, heights up
+  // to 1.5 times) pruned / whole rows are 0.965 in total time inside these limits
+  // and 1.06 outside, 1.16 there at the 95th percentile (3148^2 at 0.42 cycles a
+  // pixel, 4608 -> 8192 rows: 10.1 -> 14.5 ms).  Plans and streams clear the whole
+  // grid, a call the columns it wrote, so they go to 1.5 times and 0.7, or 1.2
+  // times and 0.8: 1632 streams 0.94 inside and 1.05 outside, 2412 plans 0.97 and
+  // 1.12 (8192^2 stream, 14000 -> 16384: 69.2 -> 58.1 ms).  In grids of up to 1024
+  // rows launches count and any height does: 2467 calls 0.996, plans 0.95 to 0.98.
   // The w planes keep the spacing of the library's height.
   g.vprune = false;
   if (g.fp32 && !pow2_v && !g.ucufft && !g.whole_rows) {
@@ -490,8 +489,8 @@ void choose_grid(GridPlan &g, double sigma_min, double sigma_max, int tile, bool
         return double(nv) <= taller * nl && width(nv) <= stored * nl;
       };
       if (!pick_nu(std::max(64.0, g.ny * bestk.sigma), vmax_px, W, nv, lm, kk) ||
-          !(pays(1.1, 0.8) || (g.resident ? pays(1.35, 0.7) : pays(1.2, 0.6)) ||
-            (nv <= 1024 && pays(1.5, 1.5))))
+          !(nv <= 1024 || (g.resident ? pays(1.2, 0.8) || pays(1.5, 0.7)
+                                      : pays(1.1, 0.8) || pays(1.2, 0.6))))
         nv = 0;
     }
     if (nv != 0 && nv < 65000 && width(nv) < double(nv)) {
