@@ -411,8 +411,8 @@ int wsg_weights_get(wsg_weights *w, double *grid, size_t *width, size_t *height,
  * weights is made or uploaded; a visibility outside the weight grid is
  * inactive.  The product is rounded to float for float weights, as
  * wsg_weights_apply stores it.  Predictions are not weighted.  w must stay
- * alive while set; NULL turns the lookup off.  Extension of the reference
- * interface. */
+ * alive while set; NULL turns the lookup off for the rows added later.
+ * Extension of the reference interface. */
 int wsg_stream_set_imaging_weights(wsg_stream *s, const wsg_weights *w);
 
 #ifdef __cplusplus
